@@ -52,10 +52,10 @@ struct Sweep {
   T hk1rc1, hk1rc3, hk2rc2;  // k1/2 * rhoc1, k1/2 * rhoc3, k2/2 * rhoc2
   T k1, k2;                  // Courant numbers dt*c/h (plain per-node scheme)
   T rhoc1, rhoc2, rhoc3;     // the material's products (plain per-node scheme)
-  // (irhoc1, irhoc2), (-irhoc1, -irhoc2), (kc1, kc2), (-kc1, -kc2): the operands of the
-  // packed FP32 x-sweep, which works on the invariant pairs (w1, w3) and (w2, w4); as
-  // aligned pairs in the kernel parameters a packed instruction takes each as one operand.
-  typename Pair<T>::type irp, nirp, kcp, nkcp;
+  // (irhoc1, irhoc2), (kc1, kc2): the operands of the packed FP32 x-sweep, which works on the
+  // invariant pairs (w1, w3) and (w2, w4); as aligned pairs in the kernel parameters a packed
+  // instruction takes each as one operand.
+  typename Pair<T>::type irp, kcp;
 };
 
 template <typename T>
@@ -67,21 +67,17 @@ struct StepConsts {
 // (x, y) pair, so a packed instruction can take it as one 8-byte operand from the kernel
 // parameters instead of a pair assembled in registers every row.
 struct YPairs {
-  float2 ir1, nir1, ir2, nir2;  // +-irhoc1, +-irhoc2
-  float2 k1, nk1, k2, nk2;      // +-kc1, +-kc2
+  float2 ir1, ir2;  // irhoc1, irhoc2
+  float2 k1, k2;    // kc1, kc2
   float2 hk1, hk2, hk1rc1, hk1rc3, hk2rc2;
 };
 
 __host__ __device__ inline YPairs make_ypairs(const Sweep<float>& c) {
   YPairs p;
   p.ir1 = make_float2(c.irhoc1, c.irhoc1);
-  p.nir1 = make_float2(-c.irhoc1, -c.irhoc1);
   p.ir2 = make_float2(c.irhoc2, c.irhoc2);
-  p.nir2 = make_float2(-c.irhoc2, -c.irhoc2);
   p.k1 = make_float2(c.kc1, c.kc1);
-  p.nk1 = make_float2(-c.kc1, -c.kc1);
   p.k2 = make_float2(c.kc2, c.kc2);
-  p.nk2 = make_float2(-c.kc2, -c.kc2);
   p.hk1 = make_float2(c.hk1, c.hk1);
   p.hk2 = make_float2(c.hk2, c.hk2);
   p.hk1rc1 = make_float2(c.hk1rc1, c.hk1rc1);
