@@ -25,7 +25,7 @@ BUILD = os.path.join(PKG, "_build")
 LIBDIR = os.path.join(PKG, "lib")
 INCLUDE = os.path.join(ROOT, "include")
 
-SOURCES = ["le2d_api.cu", "step_fused.cu", "step_split.cu", "layout.cu", "diag.cu", "batch.cu", "engine.cu",
+SOURCES = ["le2d_api.cu", "step_fused.cu", "step_split.cu", "step_tile.cu", "layout.cu", "diag.cu", "batch.cu", "engine.cu",
            "serve.cu", "diag_noalloc.cu", "slabs.cu", "selftest.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 

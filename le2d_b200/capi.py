@@ -49,6 +49,7 @@ EXPORTS = [
     "le2d_batch_autotune", "le2d_batch_autotune_reset",
     "le2d_slabs_create", "le2d_slabs_destroy", "le2d_slabs_rows", "le2d_slabs_upload",
     "le2d_slabs_download", "le2d_slabs_step_n", "le2d_slabs_wait", "le2d_selftest_ratio", "le2d_selftest_limiter", "le2d_launch_parts",
+    "le2d_block_tiles",
     "le2d_rows_out", "le2d_rows_in", "le2d_check_violations",
 ]
 
@@ -199,6 +200,7 @@ class Lib:
         L.le2d_selftest_ratio.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_longlong,
                                           ctypes.c_void_p, ctypes.c_void_p]
         L.le2d_launch_parts.argtypes = [P(self.le_task), P(ctypes.c_int)]
+        L.le2d_block_tiles.argtypes = [P(self.le_task), P(ctypes.c_int)]
         L.le2d_selftest_limiter.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_double, ctypes.c_longlong,
                                             ctypes.c_void_p]
         L.le2d_diagnostics_noalloc.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_longlong,
@@ -291,6 +293,14 @@ class Lib:
         if rc:
             raise RuntimeError(self.strerror(rc))
         return dict(zip(self.PLAN_KEYS, list(out)))
+
+    def block_tiles(self, t) -> dict:
+        """The block tiles a small grid runs on (depth 0: it runs its strip plan)."""
+        out = (ctypes.c_int * 5)()
+        rc = self.lib.le2d_block_tiles(ctypes.byref(t), out)
+        if rc:
+            raise RuntimeError(self.strerror(rc))
+        return dict(zip(("depth", "cols", "rows", "across", "down"), list(out)))
 
     def autotune(self, nx: int, ny: int):
         out = (ctypes.c_int * len(self.PLAN_KEYS))()

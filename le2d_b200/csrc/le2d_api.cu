@@ -56,9 +56,11 @@ struct DevTask {
   int method = LE2D_METHOD_FUSED;
   FusedPlan plan;
   FusedPlan plan1;  // depth-1 plan for single steps when `plan` has depth 2
-  // One le_step call held back under a two-step plan, so that the next call makes a
-  // two-step launch with it; queued by itself before anything else touches the state.
-  bool pending = false;
+  le2d::TilePlan tile;  // small grids on their default plan: several steps per launch on block tiles
+  // le_step / le_step_soa calls held back (at most one launch's steps less one), so that the
+  // following calls share a launch with them; queued before anything else touches the state.
+  int pending = 0;
+  int pending_far = 0;
   StepConsts<T> pending_c;
   long long steps = 0;
   double sim_time = 0.0;
@@ -102,11 +104,15 @@ constexpr int kMinHalvesRows = 256;  // grids with fewer rows launch whole
 // 167.7, 2048^2 131.1 / 128.7; FP64 (whole segment lengths) 2048^2 44.6 / 46.1, 4096^2 51.1 /
 // 53.7, 8192^2 55.9 / 57.2.  LE2D_HALVES=1 / 0 overrides it (on every grid of at least
 // 4 kBand rows / never).
-bool halves_for(int ny) {
+int halves_mode() {
   static const int mode = [] {  // read once, thread-safely
     const char* e = getenv("LE2D_HALVES");
     return e ? (atoi(e) != 0 ? 1 : 0) : -1;
   }();
+  return mode;
+}
+bool halves_for(int ny) {
+  const int mode = halves_mode();
   if (mode == 0 || ny < 4 * kBand) return false;
   return mode == 1 || ny >= kMinHalvesRows;
 }
@@ -226,10 +232,19 @@ int default_variant() {
   return v;
 }
 
+// Whether small grids run on block tiles by default: not when the environment asks for a
+// variant of the strip march or for its launches in halves.
+bool default_tiles() { return getenv("LE2D_FUSED_VARIANT") == nullptr && halves_mode() != 1; }
+
 // Work decomposition of the fused kernel for this task; seg_len 0 = fill the device once.
-void replan(DevTask* d, int variant, int seg_len) {
+// tiles: a small grid may run on block tiles instead (the default plan only).
+void replan(DevTask* d, int variant, int seg_len, bool tiles) {
   int dev = 0;
   cudaGetDevice(&dev);
+  d->tile = le2d::TilePlan{};
+  int sms = 0;
+  if (tiles && d->nx >= 3 && d->ny >= 3 && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
+    d->tile = le2d::plan_tiles<T>(d->nx, d->ny, sms);
   const int resident = le2d::fused_resident_warps<T>(dev, variant);
   d->halves = d->hs[0] != nullptr && halves_for(d->ny);
   le2d::FusedPlan p = le2d::plan_fused<T>(d->nx, d->ny, variant, resident, kMinSeg, d->halves);
@@ -257,6 +272,7 @@ StepConsts<T> make_consts(const le_task* t) { return le2d::make_consts(t->dt, t-
 
 struct Tuned {
   int variant = 0, seg_len = 0;
+  bool tiles = false;  // block tiles are faster than any variant
   double nu_s = 0.0;
 };
 std::mutex g_tune_mu;
@@ -305,40 +321,52 @@ int tune_size(int nx, int ny, Tuned* best) {
   le_vec2 h;
   h.x = h.y = 1;
   const StepConsts<T> c = le2d::make_consts((real)0.25, h, m);
+  // node-updates/s of the plan set, in launches of at most max_steps steps
+  auto timed = [&](int max_steps) {
+    float ms = 0.0f;
+    int steps = 0;
+    for (int k = 0; k < 2 && e == cudaSuccess; ++k)
+      e = queue_step(d, c, 0, LE2D_METHOD_FUSED, &d->cur, max_steps, &steps);
+    // estimate one launch, then time enough launches for ~3 ms
+    if (e == cudaSuccess) e = cudaEventRecord(d->ev[0], d->stream);
+    for (int k = 0; k < 3 && e == cudaSuccess; ++k)
+      e = queue_step(d, c, 0, LE2D_METHOD_FUSED, &d->cur, max_steps, &steps);
+    if (e == cudaSuccess) e = cudaEventRecord(d->ev[1], d->stream);
+    if (e == cudaSuccess) e = cudaEventSynchronize(d->ev[1]);
+    if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, d->ev[0], d->ev[1]);
+    if (e != cudaSuccess) return -1.0;
+    int reps = (int)(3.0f / (ms / 3.0f + 1e-4f));
+    reps = reps < 5 ? 5 : (reps > 400 ? 400 : reps);
+    steps = 0;
+    e = cudaEventRecord(d->ev[0], d->stream);
+    for (int k = 0; k < reps && e == cudaSuccess; ++k)
+      e = queue_step(d, c, 0, LE2D_METHOD_FUSED, &d->cur, max_steps, &steps);
+    if (e == cudaSuccess) e = cudaEventRecord(d->ev[1], d->stream);
+    if (e == cudaSuccess) e = cudaEventSynchronize(d->ev[1]);
+    if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, d->ev[0], d->ev[1]);
+    return e == cudaSuccess ? (double)nx * ny * steps / (ms * 1e-3) : -1.0;
+  };
   const int segs[] = {0, 16, 24, 32, 48, 64, 96, 128, 192, 256};
   best->nu_s = -1.0;
   for (int v = 0; v < le2d::fused_variant_count<T>() && e == cudaSuccess; ++v) {
     for (int s : segs) {
       if (s > ny) continue;
-      replan(d, v, s);
-      float ms = 0.0f;
-      int steps = 0;
-      for (int k = 0; k < 2 && e == cudaSuccess; ++k)
-        e = queue_step(d, c, 0, LE2D_METHOD_FUSED, &d->cur, 2, &steps);
-      // estimate one launch, then time enough launches for ~3 ms
-      if (e == cudaSuccess) e = cudaEventRecord(d->ev[0], d->stream);
-      for (int k = 0; k < 3 && e == cudaSuccess; ++k)
-        e = queue_step(d, c, 0, LE2D_METHOD_FUSED, &d->cur, 2, &steps);
-      if (e == cudaSuccess) e = cudaEventRecord(d->ev[1], d->stream);
-      if (e == cudaSuccess) e = cudaEventSynchronize(d->ev[1]);
-      if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, d->ev[0], d->ev[1]);
+      replan(d, v, s, false);
+      const double nus = timed(2);
       if (e != cudaSuccess) break;
-      int reps = (int)(3.0f / (ms / 3.0f + 1e-4f));
-      reps = reps < 5 ? 5 : (reps > 400 ? 400 : reps);
-      steps = 0;
-      e = cudaEventRecord(d->ev[0], d->stream);
-      for (int k = 0; k < reps && e == cudaSuccess; ++k)
-        e = queue_step(d, c, 0, LE2D_METHOD_FUSED, &d->cur, 2, &steps);
-      if (e == cudaSuccess) e = cudaEventRecord(d->ev[1], d->stream);
-      if (e == cudaSuccess) e = cudaEventSynchronize(d->ev[1]);
-      if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, d->ev[0], d->ev[1]);
-      if (e != cudaSuccess) break;
-      const double nus = (double)nx * ny * steps / (ms * 1e-3);
       if (nus > best->nu_s) {
         best->nu_s = nus;
         best->variant = v;
         best->seg_len = s;
       }
+    }
+  }
+  if (e == cudaSuccess && default_tiles()) {  // the strip plan stays the one reported (le2d_get_plan)
+    replan(d, best->variant, best->seg_len, true);
+    const double nus = d->tile.depth ? timed(d->tile.depth) : -1.0;
+    if (nus > best->nu_s) {
+      best->nu_s = nus;
+      best->tiles = true;
     }
   }
   release(d);
@@ -444,6 +472,12 @@ cudaError_t queue_step(DevTask* d, const StepConsts<T>& c, int far_rot, int meth
     return le2d::launch_split_sweep<T>(1, b, a, d->nx, d->ny, d->pitch, d->plane, c.y, c.y.k1,
                                        c.y.k2, far_rot, d->stream);
   }
+  if (d->tile.depth) {
+    const int steps = max_steps < d->tile.depth ? max_steps : d->tile.depth;
+    *cur ^= 1;
+    *done += steps;
+    return le2d::launch_tiles<T>(a, b, d->nx, d->ny, d->pitch, d->plane, c, far_rot, d->tile, steps, d->stream);
+  }
   const bool two = d->plan.depth == 2 && max_steps >= 2 && !far_rot;
   const FusedPlan& pl = two ? d->plan : d->plan1;
   if (pl.warps_per_task == 2) d->pairs_queued = true;
@@ -460,13 +494,21 @@ cudaError_t queue_step(DevTask* d, const StepConsts<T>& c, int far_rot, int meth
   return e;
 }
 
-// Queues a held-back le_step (one step) before the state is used otherwise.
+// Queues the held-back le_step calls before the state is used otherwise.
 int flush_pending(DevTask* d) {
-  if (!d->pending) return LE2D_OK;
-  d->pending = false;
-  int done = 0;
-  const cudaError_t e = queue_step(d, d->pending_c, 0, d->method, &d->cur, 1, &done);
+  const int n = d->pending;
+  d->pending = 0;
+  cudaError_t e = cudaSuccess;
+  for (int done = 0; done < n && e == cudaSuccess;)
+    e = queue_step(d, d->pending_c, d->pending_far, d->method, &d->cur, n - done, &done);
   return e == cudaSuccess ? LE2D_OK : record(d, LE2D_ECUDA, "step kernel launch", e);
+}
+
+// Steps one launch can take, for calls of one step each: consecutive calls share launches.
+int hold_steps(const DevTask* d, int far_rot) {
+  if (d->method != LE2D_METHOD_FUSED) return 1;
+  if (d->tile.depth) return d->tile.depth;
+  return far_rot ? 1 : d->plan.depth;
 }
 
 // lookup() for entry points that read, write or wait for the device state.
@@ -491,19 +533,20 @@ int run_steps(le_task* task, int nsteps, bool soa_entry, float* ms) {
   if (rc) return rc;
   const StepConsts<T> c = make_consts(task);
   const int far_rot = soa_entry ? 1 : 0;
-  // One le_step call under a two-step plan: held back, and launched as two steps together
-  // with the next call (same constants); any other use of the state queues it first.
-  if (nsteps == 1 && !soa_entry && !ms && d->method == LE2D_METHOD_FUSED && d->plan.depth == 2) {
-    if (d->pending && same_consts(d->pending_c, c)) {
-      d->pending = false;
-      int done = 0;
-      const cudaError_t e1 = queue_step(d, c, 0, d->method, &d->cur, 2, &done);
-      if (e1 != cudaSuccess) return record(d, LE2D_ECUDA, "step kernel launch", e1);
-    } else {
+  // A call of one step under a plan of several steps per launch: held back, and launched
+  // together with the following calls (same constants) once they fill a launch; any other use
+  // of the state queues it first.
+  const int hold = hold_steps(d, far_rot);
+  if (nsteps == 1 && !ms && hold > 1) {
+    if (d->pending && !(d->pending_far == far_rot && same_consts(d->pending_c, c))) {
       rc = flush_pending(d);
       if (rc) return rc;
-      d->pending = true;
-      d->pending_c = c;
+    }
+    if (d->pending == 0) d->pending_c = c;
+    d->pending_far = far_rot;
+    if (++d->pending >= hold) {
+      rc = flush_pending(d);
+      if (rc) return rc;
     }
     d->sim_time += (double)task->dt;
     d->steps += 1;
@@ -519,10 +562,11 @@ int run_steps(le_task* task, int nsteps, bool soa_entry, float* ms) {
   }
   int left = nsteps;
   // fused launches on clamped ends in halves (halves_launch) on grids tall enough
-  const bool halves = d->halves && d->method == LE2D_METHOD_FUSED && !far_rot;
+  const bool tiles = d->tile.depth > 0 && d->method == LE2D_METHOD_FUSED;
+  const bool halves = d->halves && d->method == LE2D_METHOD_FUSED && !far_rot && !tiles;
   // Long runs replay a captured graph of kGraphSteps steps (even count: buffers end where
   // they started).
-  while (left >= kGraphSteps) {
+  while (left >= kGraphSteps && !tiles) {
     const bool valid = d->graph && d->graph_cur == d->cur && d->graph_method == d->method &&
                        d->graph_far_rot == far_rot && d->graph_halves == halves &&
                        same_consts(d->graph_consts, c);
@@ -728,9 +772,9 @@ void le_init_task(le_task* task, const real dt, const le_vec2 h, const le_materi
       if (const char* st = getenv("LE2D_TEST_STALL_PAIR")) d->stall_pair = atoi(st);
       Tuned tp;
       if (tuned_plan(n.x, n.y, &tp))
-        replan(d, tp.variant, tp.seg_len);
+        replan(d, tp.variant, tp.seg_len, tp.tiles);
       else
-        replan(d, default_variant(), 0);
+        replan(d, default_variant(), 0, default_tiles());
     }
   } else {
     record(d, LE2D_ENODEV, "le_init_task");
@@ -940,7 +984,7 @@ int le2d_set_variant(le_task* task, int variant, int seg_len) {
   if (!d) return LE2D_ENOTASK;
   if (variant < -1 || variant >= le2d::fused_variant_count<T>() || seg_len < 0) return LE2D_EINVAL;
   if (!d->has_device) return LE2D_ENODEV;
-  replan(d, variant < 0 ? default_variant() : variant, seg_len);
+  replan(d, variant < 0 ? default_variant() : variant, seg_len, variant < 0 && seg_len == 0 && default_tiles());
   return LE2D_OK;
 }
 
@@ -998,7 +1042,16 @@ int le2d_launch_parts(const le_task* task, int* parts) {
   DevTask* d = lookup(task);
   if (!d) return LE2D_ENOTASK;
   if (!parts) return LE2D_EINVAL;
-  *parts = d->halves ? 3 : 1;
+  *parts = d->halves && !d->tile.depth ? 3 : 1;
+  return LE2D_OK;
+}
+
+int le2d_block_tiles(const le_task* task, int* out) {
+  DevTask* d = lookup(task);
+  if (!d) return LE2D_ENOTASK;
+  if (!out) return LE2D_EINVAL;
+  const int v[5] = {d->tile.depth, d->tile.cols, d->tile.rows, d->tile.ntx, d->tile.nty};
+  for (int k = 0; k < 5; ++k) out[k] = v[k];
   return LE2D_OK;
 }
 
@@ -1078,8 +1131,9 @@ extern "C" {
 
 int le2d_check_violations(unsigned long long* count) {
 #ifdef LE2D_CHECK
-  const unsigned long long a = le2d::check_violations_fused(), b = le2d::check_violations_batch();
-  if (count) *count = a == ~0ULL || b == ~0ULL ? ~0ULL : a + b;
+  const unsigned long long a = le2d::check_violations_fused(), b = le2d::check_violations_batch(),
+                           c = le2d::check_violations_tiles();
+  if (count) *count = a == ~0ULL || b == ~0ULL || c == ~0ULL ? ~0ULL : a + b + c;
   return 1;
 #else
   if (count) *count = 0;

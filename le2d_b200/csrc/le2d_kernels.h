@@ -70,11 +70,28 @@ cudaError_t launch_fused_rows(const T* src, T* dst, int nx, int ny, long long pi
                               const PairCtl& pair, int seg_len, int nranges, const int* lo,
                               const int* hi, cudaStream_t s);
 
+// Small grids: `depth` steps per launch on block tiles (tile.cuh, step_tile.cu).
+struct TilePlan {
+  int shape = 0;
+  int depth = 0;           // steps per launch; 0: the grid does not run on block tiles
+  int cols = 0, rows = 0;  // nodes of a tile, halo included
+  int out_x = 0;           // columns a tile writes
+  int ntx = 0, nty = 0;    // tiles across and down
+};
+// The plan of an nx x ny grid on a device of `sms` SMs.
+template <typename T>
+TilePlan plan_tiles(int nx, int ny, int sms);
+// One launch src -> dst of `steps` <= plan.depth time steps (far_rot: le_step_soa's far end).
+template <typename T>
+cudaError_t launch_tiles(const T* src, T* dst, int nx, int ny, long long pitch, long long plane,
+                         const StepConsts<T>& c, int far_rot, const TilePlan& plan, int steps, cudaStream_t s);
+
 #ifdef LE2D_CHECK
 // Bounds-checked build: accesses of the state the step kernels refused (outside the buffer),
 // on the current device, since the last call, per translation unit.
 unsigned long long check_violations_fused();
 unsigned long long check_violations_batch();
+unsigned long long check_violations_tiles();
 #endif
 
 // The plain scheme: one sweep (axis 0 = x, 1 = y) src -> dst, one thread per node, the

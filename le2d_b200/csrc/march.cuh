@@ -141,9 +141,15 @@ __device__ __forceinline__ int source_row(int m, int ny, int far_rot) {
 // zero and the division's rounding, see ratio(double)).  Face e (0..V) of the lane lies
 // between its nodes e-1 and e; the neighbour lanes supply the invariants of nodes -1 and V
 // and the fluxes of their edge nodes.
-template <int V>
-__device__ __forceinline__ void sweep_x_lane_exact(double (&f)[NF][V], const Sweep<double>& c) {
+//
+// ENDS: the lane's columns start at col0 of a grid of nx columns (block tiles, tile.cuh), and
+// the invariants and fluxes beyond the grid's ends are those of the edge column: w of every
+// column past it is the edge column's, the differences there are 0 and the fluxes equal w.
+template <int V, bool ENDS = false>
+__device__ __forceinline__ void sweep_x_lane_exact(double (&f)[NF][V], const Sweep<double>& c,
+                                                   int col0 = 0, int nx = 0) {
   constexpr unsigned kAll = 0xffffffffu;
+  const bool first = ENDS && col0 == 0, last = ENDS && col0 + V == nx;
   const double eps = tvd_eps<double>();
   double w[4][V + 2];  // nodes -1 .. V
 #pragma unroll
@@ -157,6 +163,12 @@ __device__ __forceinline__ void sweep_x_lane_exact(double (&f)[NF][V], const Swe
   for (int k = 0; k < 4; ++k) {
     w[k][0] = __shfl_up_sync(kAll, w[k][V], 1);
     w[k][V + 1] = __shfl_down_sync(kAll, w[k][1], 1);
+    if constexpr (ENDS) {
+      w[k][0] = first ? w[k][1] : w[k][0];
+#pragma unroll
+      for (int v = 1; v < V; ++v) w[k][v + 1] = col0 + v >= nx ? w[k][v] : w[k][v + 1];
+      w[k][V + 1] = last ? w[k][V] : w[k][V + 1];
+    }
   }
   double dw[4][V];
 #pragma unroll
@@ -173,7 +185,8 @@ __device__ __forceinline__ void sweep_x_lane_exact(double (&f)[NF][V], const Swe
         const double ps = psi_ratio(ex::add(d[v], eps), ex::add(d[v + 1], eps), kc);
         fl[v] = ex::add(w[k][v + 1], ex::mul(ps, d[v + 1]));
       }
-      const double f_in = __shfl_up_sync(kAll, fl[V - 1], 1);
+      double f_in = __shfl_up_sync(kAll, fl[V - 1], 1);
+      if constexpr (ENDS) f_in = first ? ex::add(w[k][1], 0.0) : f_in;  // w + psi * 0
 #pragma unroll
       for (int v = 0; v < V; ++v) dw[k][v] = ex::change(w[k][v + 1], kk, ex::sub(fl[v], v ? fl[v - 1] : f_in));
     }
@@ -187,7 +200,8 @@ __device__ __forceinline__ void sweep_x_lane_exact(double (&f)[NF][V], const Swe
         const double ps = psi_ratio(ex::sub(eps, d[v + 1]), ex::sub(eps, d[v]), kc);
         gl[v] = ex::sub(w[k][v + 1], ex::mul(ps, d[v]));
       }
-      const double g_in = __shfl_down_sync(kAll, gl[0], 1);
+      double g_in = __shfl_down_sync(kAll, gl[0], 1);
+      if constexpr (ENDS) g_in = last ? w[k][V] : g_in;
 #pragma unroll
       for (int v = 0; v < V; ++v)
         dw[k][v] = ex::change(w[k][v + 1], kk, ex::sub(gl[v], v < V - 1 ? gl[v + 1] : g_in));
@@ -298,8 +312,13 @@ __device__ __forceinline__ float2 ratio2(float2 a, float2 b) {
 // the scalar form faster.  Face e (0..V) lies between node e-1 and node e of the lane;
 // the neighbour lanes supply the fields of nodes -1 and V and the flux terms of their edge
 // nodes.
-template <int V>
-__device__ __forceinline__ void sweep_x_lane_packed(float (&f)[NF][V], const Sweep<float>& c) {
+//
+// MASK: `em[e]` (0 or 1) multiplies the differences of face e, for lanes that hold columns at
+// or beyond the grid's ends (block tiles, tile.cuh): a face with a clamped column has two equal
+// sides, so its differences are 0, and every term the neighbours take from it is then 0 too.
+template <int V, bool MASK = false>
+__device__ __forceinline__ void sweep_x_lane_packed(float (&f)[NF][V], const Sweep<float>& c,
+                                                    const float (&em)[V + 1] = {}) {
   constexpr unsigned kAll = 0xffffffffu;
   const float2 eps = f2(1e-6f, 1e-6f);
   // fields entering the x-invariants: vn = vx, sn = sxx, vt = vy, and sxy
@@ -323,6 +342,10 @@ __device__ __forceinline__ void sweep_x_lane_packed(float (&f)[NF][V], const Swe
     const float2 ds = f2(nsx - psx, nxy - pxy);
     dr[e] = fma2(neg2(ds), c.irp, dv);
     dl[e] = fma2(ds, c.irp, dv);
+    if constexpr (MASK) {
+      dr[e] = mul2(dr[e], f2(em[e], em[e]));
+      dl[e] = mul2(dl[e], f2(em[e], em[e]));
+    }
   }
   float2 na[V], b[V];  // (-A1, -A3) and (B2, B4) of node v
   {  // right-moving (w1, w3): psi_v = psi(P_v / P_{v+1}), -t_v = D_{v+1} - psi_v D_{v+1}
