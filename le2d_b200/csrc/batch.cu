@@ -355,7 +355,8 @@ cudaError_t launch_batch(const BatchInst<T>* insts, const BatchTile* tiles,
                          BatchCtl* ctl, unsigned long long wait_ns, int stall_plus1,
                          int resident_blocks, cudaStream_t s) {
   using K = BatchKernelOf<T>;
-  const int per_block = K::DEPTH == 2 ? kWarps / 2 : kWarps;  // items a block works on at once
+  constexpr int per_block = K::DEPTH == 2 ? kWarps / 2 : kWarps;  // items a block works on at once
+  static_assert(per_block == batch_block_items<T>(), "items of a block");
   long long blocks = (total_items + per_block - 1) / per_block;
   if (blocks > resident_blocks) blocks = resident_blocks;  // persistent: all blocks resident
   if (blocks < 1) blocks = 1;

@@ -137,7 +137,6 @@ template <typename T>
 int Engine<T>::set_seg_len(int rows) {
   if (rows < 1) return LE2D_EINVAL;
   seg_len_ = rows;
-  seg_set_ = true;
   return LE2D_OK;
 }
 
@@ -265,9 +264,10 @@ int Engine<T>::alloc_instance(const le2d_problem& p, Inst& in) {
   in.fail = reinterpret_cast<int*>(arena_->base() + in.state_off + sbytes);
   in.c = problem_consts<T>(p);
   // Tile height and steps per work item: explicit (autotuner trials), else the autotuner's
-  // table for the size class (LE2D_AUTOTUNE=1 tunes a class on first use), else defaults.
+  // table for the size class (LE2D_AUTOTUNE=1 tunes a class on first use), else defaults
+  // (the height chosen for each window).
   int seg = seg_len_, depth = batch_depth<T>();
-  if (!seg_set_ && !depth_set_ && use_tuned_) {
+  if (!seg_len_ && !depth_set_ && use_tuned_) {
     BatchTuned bt;
     bool have = batch_tuned(p.nx, p.ny, &bt);
     const char* a = getenv("LE2D_AUTOTUNE");
@@ -286,7 +286,6 @@ int Engine<T>::alloc_instance(const le2d_problem& p, Inst& in) {
   const int out = strip_cols(batch_lanes<T>());
   in.nstrips = (p.nx + out - 1) / out;
   in.seg_len = std::min(seg, p.ny);
-  in.nsegs = (p.ny + in.seg_len - 1) / in.seg_len;
   in.live = true;
   return LE2D_OK;
 }
@@ -388,6 +387,42 @@ int Engine<T>::read_failures(const std::vector<int>& ids) {
   return LE2D_OK;
 }
 
+// Tall tiles march fewer halo and pipeline-fill rows; short ones shorten the chain of dependent
+// items a small instance's steps are.  The height L with the least model of the window's time,
+// the larger of
+//   work:  sum over the instances of items x tiles(L) x (L + h) rows, shared by the resident
+//          tile slots, at the loaded time per row, and
+//   chain: the most items of an instance x (L + g) rows at the unloaded time per row
+// (joined by an 8-norm).  Fitted to batches of 48 instances (sides 128 to 1024, 200 to 800 steps)
+// and 24 (64 to 1024, 100 to 500) at heights of 8 to 128 rows: FP32 h = 7, 1.64 us, g = 34,
+// 0.95 us; FP64 h = 5.3, 1.49 us, g = 18, 1.05 us.  Measured (ms, 64 rows as before / the
+// height picked): FP32 48 instances 44.9 / 42.8, 24 instances 20.8 / 10.1; FP64 112.8 / 110.9
+// and 43.2 / 23.4; the 24 as requests at a server 29.4 / 16.3 and 59.7 / 36.
+template <typename T>
+int Engine<T>::window_rows(const std::vector<std::pair<int, int>>& order) const {
+  constexpr bool f32 = sizeof(T) == 4;
+  constexpr double h = f32 ? 7.0 : 5.3, loaded = f32 ? 1.64 : 1.49, g = f32 ? 34.0 : 18.0, alone = f32 ? 0.95 : 1.05;
+  const double slots = std::max(1, resident_blocks_) * (double)batch_block_items<T>();
+  constexpr int heights[] = {8, 12, 16, 24, 32, 48, 64};
+  int best = heights[0];
+  double least = 1e300;
+  for (int rows : heights) {
+    double work = 0.0, chain = 0.0;
+    for (const auto& o : order) {
+      const Inst& in = insts_[o.second];
+      const int l = std::min(in.seg_len ? in.seg_len : rows, in.p.ny);
+      work += (double)o.first * in.nstrips * ((in.p.ny + l - 1) / l) * (l + h);
+      chain = std::max(chain, o.first * (l + g));
+    }
+    const double t = std::pow(std::pow(work / slots * loaded, 8.0) + std::pow(chain * alone, 8.0), 0.125);
+    if (t < least) {
+      least = t;
+      best = rows;
+    }
+  }
+  return best;
+}
+
 template <typename T>
 typename Engine<T>::Window Engine<T>::plan_window(int window, const std::vector<long long>& done,
                                                   const std::vector<int>& cur) const {
@@ -407,8 +442,11 @@ typename Engine<T>::Window Engine<T>::plan_window(int window, const std::vector<
                      return a.first > b.first;
                    });
   int tile_base = 0;
+  const int rows = order.empty() ? 0 : window_rows(order);
   for (size_t k = 0; k < order.size(); ++k) {
     const Inst& in = insts_[order[k].second];
+    const int seg_len = std::min(in.seg_len ? in.seg_len : rows, in.p.ny);
+    const int nsegs = (in.p.ny + seg_len - 1) / seg_len;
     BatchInst<T> b;
     b.buf[0] = in.buf[0];
     b.buf[1] = in.buf[1];
@@ -421,8 +459,8 @@ typename Engine<T>::Window Engine<T>::plan_window(int window, const std::vector<
     if constexpr (std::is_same<T, float>::value) b.yq = make_ypairs(in.c.y);
     b.far_rot = in.p.stype == ST_SOA;
     b.nstrips = in.nstrips;
-    b.nsegs = in.nsegs;
-    b.seg_len = in.seg_len;
+    b.nsegs = nsegs;
+    b.seg_len = seg_len;
     b.tile_base = tile_base;
     b.parity = cur[order[k].second];
     b.steps = steps_of[order[k].second];
@@ -436,9 +474,9 @@ typename Engine<T>::Window Engine<T>::plan_window(int window, const std::vector<
     w.inst_ids.push_back(order[k].second);
     w.inst_steps.push_back(steps_of[order[k].second]);
     w.inst_items.push_back(order[k].first);
-    for (int s = 0; s < in.nsegs; ++s)
+    for (int s = 0; s < nsegs; ++s)
       for (int st = 0; st < in.nstrips; ++st) w.tiles.push_back(BatchTile{(int)k, st, s, 0});
-    tile_base += in.nstrips * in.nsegs;
+    tile_base += in.nstrips * nsegs;
   }
   w.steps = order.empty() ? 0 : order.front().first;
   w.step_items.assign(w.steps + 1, 0);

@@ -49,7 +49,8 @@ class Engine {
     int cur = 0;    // buffer holding the current state
     int depth = 1;  // steps per work item of the batched kernel
     StepConsts<T> c;
-    int nstrips = 0, nsegs = 0, seg_len = 0;
+    int nstrips = 0;
+    int seg_len = 0;  // tile height; 0: chosen for each window (window_rows)
     bool live = false;
     int* fail = nullptr;     // failure word on the device (in the instance's arena block)
     bool failed = false;     // a dependency wait of one of its tiles gave up: no results
@@ -104,14 +105,12 @@ class Engine {
   void set_wait_ns(unsigned long long ns) { wait_ns_ = ns; }
   // Tile height and steps per work item for instances added afterwards (the autotuner's
   // trials); otherwise they come from the autotuner's table for the instance's size class,
-  // or the defaults (64 rows, batch_depth<T>()).
+  // or the defaults (a height chosen for each window, batch_depth<T>()).
   int set_seg_len(int rows);
   int set_depth(int depth);
   // Whether instances added afterwards take their tiles from the autotuner's table (default)
   // or the defaults.  The serving loop uses the defaults: the table is tuned for throughput
-  // on a full batch, and its taller tiles lengthen each small instance's chain of steps
-  // (measured: untuned p50 latency 0.22 s against 0.39 s at 10 requests/s, and 46 against
-  // 43 solves/s at 200).
+  // on a full batch, and its taller tiles lengthen each small instance's chain of steps.
   void set_use_tuned(bool on) { use_tuned_ = on; }
   size_t arena_used() const { return arena_ ? arena_->used() : 0; }
   size_t arena_capacity() const { return arena_ ? arena_->capacity() : 0; }
@@ -130,6 +129,9 @@ class Engine {
   // done_steps / cur: each instance's steps so far and current buffer before the window.
   Window plan_window(int window, const std::vector<long long>& done_steps,
                      const std::vector<int>& cur) const;
+  // Tile height of the instances without one of their own, for a window in which instance
+  // order[k].second runs order[k].first work items.
+  int window_rows(const std::vector<std::pair<int, int>>& order) const;
   int ensure_scratch(size_t insts, size_t tiles, size_t items, size_t done, size_t ctls);
   int launch_window(const Window& w, size_t inst_off, size_t tile_off, size_t item_off,
                     size_t done_off, size_t ctl_off);
@@ -147,8 +149,7 @@ class Engine {
   unsigned long long wait_ns_ = 2000000000ULL;
   int stall_tile_ = -1;  // test hook from LE2D_TEST_STALL_TILE (see launch_batch): in the
                          // engine's first window only
-  int seg_len_ = 64;
-  bool seg_set_ = false;
+  int seg_len_ = 0;  // explicit tile height (set_seg_len)
   int depth_set_ = 0;
   bool use_tuned_ = true;
   int resident_blocks_ = 0;

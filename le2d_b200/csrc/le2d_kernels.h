@@ -167,6 +167,9 @@ template <typename T>
 size_t batch_smem();
 template <typename T>
 int batch_resident_blocks(int device);
+// Work items a block of the batched kernel has in hand at once.
+template <typename T>
+constexpr int batch_block_items() { return sizeof(T) == 4 ? 2 : 4; }
 // step_items[r] = work items before window item step r (r = 0..nsteps; an item step
 // advances each instance by its depth); done[] and ctl zeroed.
 // stall_plus1 > 0 is a test hook: tile (stall_plus1 - 1) never publishes its first step,
