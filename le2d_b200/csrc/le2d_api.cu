@@ -64,11 +64,14 @@ struct DevTask {
   StepConsts<T> pending_c;
   long long steps = 0;
   double sim_time = 0.0;
-  // CUDA graph of kGraphSteps steps starting from buffer graph_cur.
-  cudaGraphExec_t graph = nullptr;
-  int graph_cur = -1, graph_method = -1, graph_far_rot = -1;
+  // CUDA graphs of kGraphSteps steps from either buffer, for runs of more than kDirectSteps
+  // steps of one kind (method, far end, halves, constants); direct_steps: steps of the
+  // current kind launched without them so far.
+  cudaGraphExec_t graph[2] = {nullptr, nullptr};
+  int graph_method = -1, graph_far_rot = -1;
   bool graph_halves = false;
   StepConsts<T> graph_consts;
+  long long direct_steps = 0;
   // Fused launches in halves (halves_launch): hs[0] the band of rows around the middle of
   // the grid (high priority), hs[1] / hs[2] the rows above / below it; hev[i][k & 1] after
   // stream i's part of launch k of the current sequence, hk launches so far.
@@ -80,6 +83,12 @@ struct DevTask {
 };
 
 constexpr int kGraphSteps = 64;  // even, so a replay leaves the current buffer unchanged
+// Steps launched one by one before a graph is captured.  A replayed step saves about 1.2 us
+// (2048^2 FP32: 33.3 against 31.0 us a step), a capture costs 2 to 4 ms, so it pays after some
+// two thousand steps; a caller that comes back for more steps gets it after its first 512.
+// The first 128 steps of a new task then take 3.2 ms (1500 x 1400), 4.3 ms (2048^2) and 5.0 ms
+// (3001 x 1777) where capturing at once took 5.3, 6.2 and 7.0 ms.
+constexpr long long kDirectSteps = 512;
 // Bound of every wait between the two warps of a warp-pair tile (they share a block, so a
 // wait that long means a fault in the kernel, not a slow partner).
 constexpr unsigned long long kPairWaitNs = 1000000000ull;
@@ -236,6 +245,14 @@ int default_variant() {
 // variant of the strip march or for its launches in halves.
 bool default_tiles() { return getenv("LE2D_FUSED_VARIANT") == nullptr && halves_mode() != 1; }
 
+void drop_graphs(DevTask* d) {
+  for (cudaGraphExec_t& g : d->graph) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
+  d->direct_steps = 0;
+}
+
 // Work decomposition of the fused kernel for this task; seg_len 0 = fill the device once.
 // tiles: a small grid may run on block tiles instead (the default plan only).
 void replan(DevTask* d, int variant, int seg_len, bool tiles) {
@@ -261,8 +278,7 @@ void replan(DevTask* d, int variant, int seg_len, bool tiles) {
     const int v = sizeof(T) == 4 ? 2 : 15;  // the fastest one-step variant
     d->plan1 = le2d::plan_fused<T>(d->nx, d->ny, v, le2d::fused_resident_warps<T>(dev, v), kMinSeg);
   }
-  if (d->graph) cudaGraphExecDestroy(d->graph);
-  d->graph = nullptr;
+  drop_graphs(d);
 }
 
 // Step constants from the task as it is now (the caller may change dt between steps).
@@ -518,6 +534,27 @@ DevTask* lookup_sync(const le_task* task) {
   return d;
 }
 
+// A graph of kGraphSteps steps from the current buffer.
+int capture_steps(DevTask* d, const StepConsts<T>& c, int far_rot, bool halves, cudaGraphExec_t* exec) {
+  cudaGraph_t g = nullptr;
+  cudaError_t e = cudaStreamBeginCapture(d->stream, cudaStreamCaptureModeThreadLocal);
+  if (e != cudaSuccess) return record(d, LE2D_ECUDA, "graph capture", e);
+  int cur = d->cur;
+  if (halves) e = halves_begin(d);
+  for (int s = 0; s < kGraphSteps && e == cudaSuccess;)
+    e = queue_step(d, c, far_rot, d->method, &cur, kGraphSteps - s, &s, halves);
+  if (halves && e == cudaSuccess) e = halves_end(d);
+  const cudaError_t e2 = cudaStreamEndCapture(d->stream, &g);
+  if (e != cudaSuccess || e2 != cudaSuccess) {
+    if (g) cudaGraphDestroy(g);
+    return record(d, LE2D_ECUDA, "graph capture", e != cudaSuccess ? e : e2);
+  }
+  e = cudaGraphInstantiate(exec, g, 0);
+  cudaGraphDestroy(g);
+  if (e != cudaSuccess) *exec = nullptr;
+  return e == cudaSuccess ? LE2D_OK : record(d, LE2D_ECUDA, "graph instantiate", e);
+}
+
 int run_steps(le_task* task, int nsteps, bool soa_entry, float* ms) {
   DevTask* d = lookup(task);
   if (!d) {
@@ -564,52 +601,45 @@ int run_steps(le_task* task, int nsteps, bool soa_entry, float* ms) {
   // fused launches on clamped ends in halves (halves_launch) on grids tall enough
   const bool tiles = d->tile.depth > 0 && d->method == LE2D_METHOD_FUSED;
   const bool halves = d->halves && d->method == LE2D_METHOD_FUSED && !far_rot && !tiles;
-  // Long runs replay a captured graph of kGraphSteps steps (even count: buffers end where
-  // they started).
-  while (left >= kGraphSteps && !tiles) {
-    const bool valid = d->graph && d->graph_cur == d->cur && d->graph_method == d->method &&
-                       d->graph_far_rot == far_rot && d->graph_halves == halves &&
-                       same_consts(d->graph_consts, c);
-    if (!valid) {
-      if (d->graph) cudaGraphExecDestroy(d->graph);
-      d->graph = nullptr;
-      cudaGraph_t g = nullptr;
-      e = cudaStreamBeginCapture(d->stream, cudaStreamCaptureModeThreadLocal);
-      if (e != cudaSuccess) return record(d, LE2D_ECUDA, "graph capture", e);
-      int cur = d->cur;
-      if (halves) e = halves_begin(d);
-      for (int s = 0; s < kGraphSteps && e == cudaSuccess;)
-        e = queue_step(d, c, far_rot, d->method, &cur, kGraphSteps - s, &s, halves);
-      if (halves && e == cudaSuccess) e = halves_end(d);
-      cudaError_t e2 = cudaStreamEndCapture(d->stream, &g);
-      if (e != cudaSuccess || e2 != cudaSuccess)
-        return record(d, LE2D_ECUDA, "graph capture", e != cudaSuccess ? e : e2);
-      e = cudaGraphInstantiate(&d->graph, g, 0);
-      cudaGraphDestroy(g);
-      if (e != cudaSuccess) return record(d, LE2D_ECUDA, "graph instantiate", e);
-      d->graph_cur = d->cur;
-      d->graph_method = d->method;
-      d->graph_far_rot = far_rot;
-      d->graph_halves = halves;
-      d->graph_consts = c;
-    }
-    e = cudaGraphLaunch(d->graph, d->stream);
-    if (e != cudaSuccess) return record(d, LE2D_ECUDA, "graph launch", e);
-    left -= kGraphSteps;
+  if (!(d->graph_method == d->method && d->graph_far_rot == far_rot && d->graph_halves == halves &&
+        same_consts(d->graph_consts, c))) {
+    drop_graphs(d);
+    d->graph_method = d->method;
+    d->graph_far_rot = far_rot;
+    d->graph_halves = halves;
+    d->graph_consts = c;
   }
-  if (left > 0 && halves) {
-    e = halves_begin(d);
-    if (e != cudaSuccess) return record(d, LE2D_ECUDA, "step kernel launch", e);
-  }
+  // Long runs replay a captured graph of kGraphSteps steps (even count: buffers end where they
+  // started), one for each buffer a run may start from: an odd number of launches between two
+  // replays used to capture it again, 4 ms a call.
   while (left > 0) {
-    int done = 0;
-    e = queue_step(d, c, far_rot, d->method, &d->cur, left, &done, halves);
-    if (e != cudaSuccess) return record(d, LE2D_ECUDA, "step kernel launch", e);
-    left -= done;
-    if (left == 0 && halves) {
-      e = halves_end(d);
-      if (e != cudaSuccess) return record(d, LE2D_ECUDA, "step kernel launch", e);
+    if (!tiles && left >= kGraphSteps && d->direct_steps >= kDirectSteps) {
+      cudaGraphExec_t& graph = d->graph[d->cur];
+      if (!graph) {
+        rc = capture_steps(d, c, far_rot, halves, &graph);
+        if (rc) return rc;
+      }
+      e = cudaGraphLaunch(graph, d->stream);
+      if (e != cudaSuccess) return record(d, LE2D_ECUDA, "graph launch", e);
+      left -= kGraphSteps;
+      continue;
     }
+    int direct = left;
+    if (!tiles && left >= kGraphSteps && d->direct_steps + left > kDirectSteps) {
+      direct = (int)(kDirectSteps - d->direct_steps);
+      direct += direct & 1;
+      if (direct > left) direct = left;
+    }
+    left -= direct;
+    d->direct_steps += direct;
+    if (halves) e = halves_begin(d);
+    while (direct > 0 && e == cudaSuccess) {
+      int done = 0;
+      e = queue_step(d, c, far_rot, d->method, &d->cur, direct, &done, halves);
+      direct -= done;
+    }
+    if (halves && e == cudaSuccess) e = halves_end(d);
+    if (e != cudaSuccess) return record(d, LE2D_ECUDA, "step kernel launch", e);
   }
   if (ms) {
     e = cudaEventRecord(d->ev[1], d->stream);
@@ -627,7 +657,7 @@ int run_steps(le_task* task, int nsteps, bool soa_entry, float* ms) {
 }
 
 void release(DevTask* d) {
-  if (d->graph) cudaGraphExecDestroy(d->graph);
+  drop_graphs(d);
   destroy_halves(d);
   if (d->ev[0]) cudaEventDestroy(d->ev[0]);
   if (d->ev[1]) cudaEventDestroy(d->ev[1]);
