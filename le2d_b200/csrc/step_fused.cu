@@ -361,6 +361,13 @@ constexpr int kWaves = 8;
 //   waves of one half, h = 8, beta = 0, alpha = 0.2, kappa = 0.1 -- the fastest measured length
 //   on each (2-3 % above the whole launches' lengths in halves: 8192^2 58.8 against 57.3,
 //   2048^2 48.1 against 46.5 Gnu/s).
+// Where a warp-pair model picks its shortest length, 32 rows, the grid has too few tiles to fill
+// the device and its launch lasts as long as one tile's rows march: shorter segments end sooner.
+// Two more models choose those, fitted on 1200 x 900 to 3001 x 1777 with segments of 8 to 48
+// rows: in halves h = 18, beta = 0.5, alpha = 0 (within 0.5 % of the fastest measured length on
+// each), whole h = 6, beta = 0, alpha = 0.5 (the fastest on each).  us a step in halves at 32
+// rows / at the length picked: 2048 x 1024 23.7 / 19.1, 1500^2 26.4 / 20.7, 2050 x 1500 27.0 / 24.4,
+// 4000 x 1000 30.2 / 27.6, 2048^2 31.0 / 29.9; whole, 2048 x 1024 22.7 / 18.6.
 struct SegModel {
   double h, beta, alpha, kappa;
   const int* lens;
@@ -370,6 +377,9 @@ constexpr int kPairLens[] = {32, 48, 64, 80, 96, 128, 160, 192, 256};
 constexpr int kStepLensF64[] = {16, 24, 32, 40, 48, 56, 64, 80, 96, 112, 128};
 constexpr SegModel kPairModel{10.0, 0.1, 0.5, 0.02, kPairLens, 9};
 constexpr SegModel kPairHalvesModel{14.0, 0.0, 0.2, 0.0, kPairLens, 9};
+constexpr int kShortLens[] = {8, 10, 12, 16, 20, 24, 28, 32};
+constexpr SegModel kPairShortModel{6.0, 0.0, 0.5, 0.0, kShortLens, 8};
+constexpr SegModel kPairShortHalvesModel{18.0, 0.5, 0.0, 0.0, kShortLens, 8};
 constexpr SegModel kStepModelF64{8.0, 0.3, 0.0, 0.1, kStepLensF64, 11};
 constexpr int kStepHalvesLensF64[] = {16, 24, 32, 48, 64, 96, 128};
 constexpr SegModel kStepHalvesModelF64{8.0, 0.0, 0.2, 0.1, kStepHalvesLensF64, 7};
@@ -405,11 +415,13 @@ FusedPlan plan_fused(int nx, int ny, int variant, int resident_warps, int min_se
   if (target < 1) target = 1;
   int seg = (ny + target - 1) / target;
   if (seg < min_seg * pl.depth) seg = min_seg * pl.depth;
-  if (resident_tasks > 0 && pl.warps_per_task == 2 && halves)  // each half's waves
-    seg = model_segment(kPairHalvesModel, ny, pl.nstrips, 2 * resident_tasks, min_seg * pl.depth);
-  else if (resident_tasks > 0 && pl.warps_per_task == 2)
-    seg = model_segment(kPairModel, ny, pl.nstrips, resident_tasks, min_seg * pl.depth);
-  else if (resident_tasks > 0 && sizeof(T) == 8 && pl.depth == 1 && halves)
+  if (resident_tasks > 0 && pl.warps_per_task == 2) {
+    const int tiles = halves ? 2 * resident_tasks : resident_tasks;  // in halves: each half's waves
+    seg = model_segment(halves ? kPairHalvesModel : kPairModel, ny, pl.nstrips, tiles, min_seg * pl.depth);
+    if (seg <= kPairLens[0])
+      seg = model_segment(halves ? kPairShortHalvesModel : kPairShortModel, ny, pl.nstrips, tiles, kShortLens[0]);
+  }
+  if (resident_tasks > 0 && sizeof(T) == 8 && pl.depth == 1 && halves)
     seg = model_segment(kStepHalvesModelF64, ny, pl.nstrips, 2 * resident_tasks, min_seg);
   else if (resident_tasks > 0 && sizeof(T) == 8 && pl.depth == 1)
     seg = model_segment(kStepModelF64, ny, pl.nstrips, resident_tasks, min_seg);
