@@ -70,7 +70,7 @@ int le2d_set_method(le_task *task, int method);
 /* Fused-kernel variant (columns per lane / register bound / input-ring depth / temporal-block
  * depth / warp pair; -1 = default) and row segment length (0 = the planner's) for this
  * task's grid.  A variant of temporal-block depth 2 advances two steps per launch; odd step
- * counts and le_step_soa then take single steps.  On a warp-pair variant a wait between the
+ * counts, and le_step_soa on a variant without warp pairs, then take single steps.  On a warp-pair variant a wait between the
  * two warps of a tile that runs out (a fault, not a slow partner) is reported as
  * LE2D_ETIMEOUT at the next synchronisation (le2d_wait, le2d_download, le2d_sync_host). */
 int le2d_set_variant(le_task *task, int variant, int seg_len);

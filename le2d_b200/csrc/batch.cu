@@ -27,9 +27,9 @@
 // (march_pair.cuh): the producer claims the item, passes its index to the consumer through
 // the pair's queue, waits for the item's dependencies, reads the state and runs the first
 // step; the consumer runs the second step on the rows it is handed, writes them, records
-// receiver samples and publishes the tile.  The last item of an odd step count, and every
-// item of an le_step_soa instance, advances one step: the consumer writes the producer's
-// rows as they are.
+// receiver samples and publishes the tile.  The last item of an odd step count advances
+// one step: the consumer writes the producer's rows as they are.  (le_step_soa's far end reads
+// step A's rows down to ny-7, within the tile above the last one: tiles are at least 8 rows.)
 // A producer may claim its next item while its consumer still finishes the last one: all
 // rows of that item are already in the queue, so the consumer finishes without it.
 // The x-sweep runs one invariant at a time (sweep_x_lane_diff), which at this kernel's
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB)
       const int y0 = bt.seg * I.seg_len;
       const int y1 = min(y0 + I.seg_len, I.ny);
       const ItemConsts<T>& k = load_item_consts(kslot, I);
-      if (!march::pair_produce<T, V, kNpf, true, false>(g, k.x, k.y, bt.strip, y0, y1, smem, bars, wait_ns,
+      if (!march::pair_produce<T, V, kNpf, true, true, false>(g, k.x, k.y, bt.strip, y0, y1, smem, bars, wait_ns,
                                                         status, u, nadv == 1))
         break;
     }
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB)
         tap_b = march::RowTap<T>{I.trace + ((before + 2) / I.trace_every - 1) * 2 * I.pitch, I.trace_row};
       const int tile_id = I.tile_base + bt.seg * I.nstrips + bt.strip;
       const ItemConsts<T>& k = load_item_consts(kslot, I);
-      if (!march::pair_consume<T, V, kNpf, true, false>(g, k.x, k.y, bt.strip, y0, y1, smem, bars, wait_ns,
+      if (!march::pair_consume<T, V, kNpf, true, true, false>(g, k.x, k.y, bt.strip, y0, y1, smem, bars, wait_ns,
                                                         status, u, nadv == 1, tap_a, tap_b))
         break;
       __syncwarp();  // the consumer wrote the tile's new state and publishes it

@@ -278,8 +278,7 @@ int Engine<T>::alloc_instance(const le2d_problem& p, Inst& in) {
     }
   }
   if (depth_set_) depth = std::min(depth_set_, batch_depth<T>());
-  // le_step_soa's far end is not a clamp: its instances advance one step per work item
-  in.depth = p.stype == ST_AOS ? depth : 1;
+  in.depth = depth;
   // one- and two-step tiles have the same strips at the two-step kernel's 4 columns per
   // lane (one halo lane per side for either)
   static_assert(strip_cols(4) == strip_cols2(4), "strip widths of one and two steps");

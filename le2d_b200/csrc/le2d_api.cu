@@ -102,7 +102,8 @@ constexpr unsigned long long kPairWaitNs = 1000000000ull;
 // So the upper and lower parts run on streams of their own and overlap each other's ends,
 // as the row slabs of two devices do (slabs.cu), without copies: the parts share the
 // task's buffers and write disjoint rows.  The stencil of a launch reaches 4 rows (two
-// steps of two), so kBand = 4.  Bitwise the same results as whole launches.
+// steps of two), so kBand = 4; le_step_soa's last rows read rows ny-7 and below, which lie in
+// the lower part or the band too (ny >= 4 kBand).  Bitwise the same results as whole launches.
 constexpr int kBand = 4;
 constexpr int kMinHalvesRows = 256;  // grids with fewer rows launch whole
 
@@ -170,7 +171,7 @@ cudaError_t halves_end(DevTask* d) {
 
 // Launch k of the sequence, from a into b, in three parts.
 cudaError_t halves_launch(DevTask* d, const T* a, T* b, const StepConsts<T>& c, const FusedPlan& pl,
-                          const le2d::PairCtl& pc) {
+                          int far_rot, const le2d::PairCtl& pc) {
   const long long k = d->hk;
   const int mid = d->ny / 2;
   const int lo[3] = {mid - kBand, 0, mid + kBand}, hi[3] = {mid + kBand, mid - kBand, d->ny};
@@ -180,13 +181,13 @@ cudaError_t halves_launch(DevTask* d, const T* a, T* b, const StepConsts<T>& c, 
     if (e == cudaSuccess) e = cudaStreamWaitEvent(d->hs[0], d->hev[2][(k + 1) & 1], 0);
   }
   if (e == cudaSuccess)
-    e = le2d::launch_fused_rows<T>(a, b, d->nx, d->ny, d->pitch, d->plane, c, 0, pl, pc, 2 * kBand, 1, &lo[0],
+    e = le2d::launch_fused_rows<T>(a, b, d->nx, d->ny, d->pitch, d->plane, c, far_rot, pl, pc, 2 * kBand, 1, &lo[0],
                                    &hi[0], d->hs[0]);
   if (e == cudaSuccess) e = cudaEventRecord(d->hev[0][k & 1], d->hs[0]);
   for (int i = 1; i < 3 && e == cudaSuccess; ++i) {  // each interior part after the band of launch k-1
     if (k > 0) e = cudaStreamWaitEvent(d->hs[i], d->hev[0][(k + 1) & 1], 0);
     if (e == cudaSuccess)
-      e = le2d::launch_fused_rows<T>(a, b, d->nx, d->ny, d->pitch, d->plane, c, 0, pl, pc, pl.seg_len, 1, &lo[i],
+      e = le2d::launch_fused_rows<T>(a, b, d->nx, d->ny, d->pitch, d->plane, c, far_rot, pl, pc, pl.seg_len, 1, &lo[i],
                                      &hi[i], d->hs[i]);
     if (e == cudaSuccess) e = cudaEventRecord(d->hev[i][k & 1], d->hs[i]);
   }
@@ -274,7 +275,7 @@ void replan(DevTask* d, int variant, int seg_len, bool tiles) {
   }
   d->plan = p;
   d->plan1 = p;
-  if (p.depth != 1) {  // odd remainders and le_step_soa run single steps
+  if (p.depth != 1) {  // odd remainders, and le_step_soa without warp pairs, run single steps
     const int v = sizeof(T) == 4 ? 2 : 15;  // the fastest one-step variant
     d->plan1 = le2d::plan_fused<T>(d->nx, d->ny, v, le2d::fused_resident_warps<T>(dev, v), kMinSeg);
   }
@@ -471,11 +472,17 @@ int ensure_host_current(DevTask* d, le_task* task) {
   return LE2D_OK;
 }
 
+// Steps a launch of the strip march can take: two under a plan of temporal-block depth 2, on
+// le_step_soa's far end only where warp pairs march it.
+int strip_steps(const DevTask* d, int far_rot) {
+  return d->plan.depth == 2 && (!far_rot || d->plan.warps_per_task == 2) ? 2 : 1;
+}
+
 // Queues one launch of at most max_steps (>= 1) steps from buf[cur] and adds the steps it
-// makes to *done (halves: a fused launch on clamped ends goes in halves, inside a sequence
-// that halves_begin opened).  The fused kernel writes buf[cur^1] and flips cur -- two steps when the
-// plan has temporal-block depth 2 and two are wanted (clamped ends only), else one; the
-// split scheme sweeps x into buf[cur^1] and y back into buf[cur].
+// makes to *done (halves: a fused launch goes in halves, inside a sequence that halves_begin
+// opened).  The fused kernel writes buf[cur^1] and flips cur -- two steps where strip_steps()
+// allows and two are wanted, else one; the split scheme sweeps x into buf[cur^1] and y back
+// into buf[cur].
 cudaError_t queue_step(DevTask* d, const StepConsts<T>& c, int far_rot, int method, int* cur,
                        int max_steps, int* done, bool halves) {
   T* a = d->buf[*cur];
@@ -494,15 +501,15 @@ cudaError_t queue_step(DevTask* d, const StepConsts<T>& c, int far_rot, int meth
     *done += steps;
     return le2d::launch_tiles<T>(a, b, d->nx, d->ny, d->pitch, d->plane, c, far_rot, d->tile, steps, d->stream);
   }
-  const bool two = d->plan.depth == 2 && max_steps >= 2 && !far_rot;
+  const bool two = max_steps >= 2 && strip_steps(d, far_rot) == 2;
   const FusedPlan& pl = two ? d->plan : d->plan1;
   if (pl.warps_per_task == 2) d->pairs_queued = true;
   le2d::PairCtl pc;
   pc.status = d->d_status;
   pc.wait_ns = kPairWaitNs;
   pc.stall_task = d->stall_pair;
-  cudaError_t e = halves && !far_rot
-                      ? halves_launch(d, a, b, c, pl, pc)
+  cudaError_t e = halves
+                      ? halves_launch(d, a, b, c, pl, far_rot, pc)
                       : le2d::launch_fused_step<T>(a, b, d->nx, d->ny, d->pitch, d->plane, c, far_rot, pl, pc,
                                                    d->stream);
   *cur ^= 1;
@@ -524,7 +531,7 @@ int flush_pending(DevTask* d) {
 int hold_steps(const DevTask* d, int far_rot) {
   if (d->method != LE2D_METHOD_FUSED) return 1;
   if (d->tile.depth) return d->tile.depth;
-  return far_rot ? 1 : d->plan.depth;
+  return strip_steps(d, far_rot);
 }
 
 // lookup() for entry points that read, write or wait for the device state.
@@ -598,9 +605,9 @@ int run_steps(le_task* task, int nsteps, bool soa_entry, float* ms) {
     if (e != cudaSuccess) return record(d, LE2D_ECUDA, "event record", e);
   }
   int left = nsteps;
-  // fused launches on clamped ends in halves (halves_launch) on grids tall enough
+  // fused launches in halves (halves_launch) on grids tall enough
   const bool tiles = d->tile.depth > 0 && d->method == LE2D_METHOD_FUSED;
-  const bool halves = d->halves && d->method == LE2D_METHOD_FUSED && !far_rot && !tiles;
+  const bool halves = d->halves && d->method == LE2D_METHOD_FUSED && !tiles;
   if (!(d->graph_method == d->method && d->graph_far_rot == far_rot && d->graph_halves == halves &&
         same_consts(d->graph_consts, c))) {
     drop_graphs(d);

@@ -55,7 +55,7 @@ struct PairCtl {
 };
 
 // One fused launch src -> dst: plan.depth time steps.  far_rot selects the le_step_soa
-// far-end rows (depth-1 plans only).
+// far-end rows (one-step and warp-pair plans).
 template <typename T>
 cudaError_t launch_fused_step(const T* src, T* dst, int nx, int ny, long long pitch,
                               long long plane, const StepConsts<T>& c, int far_rot,
@@ -159,8 +159,8 @@ struct BatchCtl {
 
 template <typename T>
 int batch_lanes();
-// Temporal-block depth of the batched kernel for clamped-end (le_step) instances: 2 for
-// FP32 (producer / consumer warp pairs), 1 for FP64; le_step_soa instances use 1.
+// Temporal-block depth of the batched kernel: 2 for FP32 (producer / consumer warp pairs), 1
+// for FP64.
 template <typename T>
 int batch_depth();
 template <typename T>

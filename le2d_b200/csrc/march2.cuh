@@ -16,7 +16,7 @@
 // warp shuffles; and at a row outside [0, ny) the edge row's, so the pseudo rows step A
 // produces above row 0 / below row ny-1 are dropped and rows 0 / ny-1 are fed to step B
 // once for every row of its stencil that they stand for.  (le_step_soa's far end is not a
-// clamp; SoA tasks use single steps.)
+// clamp; warp pairs know it (march_pair.cuh), the one-warp tiles here do not.)
 #pragma once
 
 #include "march.cuh"

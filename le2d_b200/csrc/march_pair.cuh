@@ -21,8 +21,15 @@
 // [xs+4, xs+32V-4); the producer overwrites step A's values outside [0, nx) with the edge
 // column's and hands row 0 / ny-1 over once and the consumer feeds it to step B once for
 // every row of its stencil it stands for (the same count both warps compute).  A one-step
-// tile (in the batched kernel: an odd last step, or le_step_soa's far end) hands over step
-// A's own rows [y0, y1), which the consumer writes as they are.
+// tile (in the batched kernel: an odd last step) hands over step A's own rows [y0, y1), which
+// the consumer writes as they are.
+//
+// le_step_soa's far end (g.far_rot): the rows step B reads past ny-1 are step A's rows ny-5 and
+// ny-4 (clamped at 0), long out of the rings when they are needed.  The producer of a tile that
+// reads them marches those few rows again -- six rows in the last tile of a strip -- and hands
+// them over after row ny-1.  FAR compiles that in; the single-solve kernels leave it out for
+// le_step grids, whose loops it slowed by 0.6 to 1.7 %.  le_step_soa, single steps before / now
+// (us a step, in halves): 2050 x 1500 28.4 / 25.2, 2048^2 35.0 / 30.5, 4096^2 122.7 / 90.5.
 #pragma once
 
 #include "march2.cuh"
@@ -108,13 +115,15 @@ static_assert(pair_smem_bytes<float, 4, 2>() % 16 == 0 && pair_smem_bytes<double
               "pair shared memory must keep 16-byte alignment");
 
 // How many rows of step B's stencil step-A row ka stands for (tile rows [y0, y1)):
-// step B reads rows [y0-2, y1+2) clamped to [0, ny).  A one-step tile hands over its own
-// rows [y0, y1) only, once each.
-__device__ __forceinline__ int row_uses(int ka, int y0, int y1, int ny, bool one_step = false) {
+// step B reads rows [y0-2, y1+2) clamped to [0, ny); with le_step_soa's far end the rows past
+// ny-1 are handed over by themselves.  A one-step tile hands over its own rows [y0, y1) only,
+// once each.
+__device__ __forceinline__ int row_uses(int ka, int y0, int y1, int ny, bool one_step, bool far_rot) {
   if (one_step) return ka >= y0 && ka < y1 ? 1 : 0;
-  int reps = ka < 0 || ka >= ny ? 0 : 1;
+  if (ka >= ny) return far_rot ? 1 : 0;
+  int reps = ka < 0 ? 0 : 1;
   if (ka == 0 && y0 < 2) reps += 2 - y0;
-  if (ka == ny - 1 && y1 + 2 > ny) reps += y1 + 2 - ny;
+  if (!far_rot && ka == ny - 1 && y1 + 2 > ny) reps += y1 + 2 - ny;
   return reps;
 }
 
@@ -348,9 +357,9 @@ __device__ __forceinline__ void march_tile_interior(const GridRef<T>& g, const S
 
 // Producer warp: step A of strip `strip`, rows [y0, y1) of the tile, handing its rows to
 // the consumer; `u` counts the queue's handoffs (it continues across tiles).  A one_step
-// tile (an odd last step, or le_step_soa's far end, which g.far_rot selects) hands over
-// step A's rows [y0, y1) only, which the consumer writes.  Returns false if a wait gave up.
-template <typename T, int V, int NPF, bool COHERENT, bool XPACK = true, typename CY = Sweep<T>>
+// tile (an odd last step) hands over step A's rows [y0, y1) only, which the consumer writes.
+// Returns false if a wait gave up.
+template <typename T, int V, int NPF, bool COHERENT, bool FAR, bool XPACK = true, typename CY = Sweep<T>>
 __device__ __forceinline__ bool pair_produce(const GridRef<T>& g, const Sweep<T>& cx, const CY& cy, int strip,
                                              int y0, int y1, T* smem_pair,
                                              unsigned long long* bars,
@@ -372,56 +381,72 @@ __device__ __forceinline__ bool pair_produce(const GridRef<T>& g, const Sweep<T>
   const int xs = strip * kOut - H2 * V;
   const int col0 = xs + lane * V;
   const bool interior = xs >= 0 && xs + kIn <= g.nx;
-  const int mend = one_step ? y1 + 2 : y1 + 4;  // one step needs the raw rows up to y1+1 only
 
   YPipe<T, V> ya;
-  ya.init();
-#pragma unroll
-  for (int k = 0; k < NF; ++k) *reinterpret_cast<VT*>(a_ring + 2 * kRow + k * kIn) = VT{};
-#pragma unroll
-  for (int j = 0; j < NPF - 1; ++j)
-    fetch_row<T, V, COHERENT>(in_ring + j * kRow, g, source_row(y0 - 4 + j, g.ny, g.far_rot), col0,
-                              interior);
-  int islot = 0, aslot = 0;
   bool ok = true;
-  for (int m = y0 - 4; m < mend; ++m) {
-    {
-      const int mm = m + NPF - 1;
-      const int ns = islot + NPF - 1 >= NPF ? islot - 1 : islot + NPF - 1;
-      if (mm < mend)
-        fetch_row<T, V, COHERENT>(in_ring + ns * kRow, g, source_row(mm, g.ny, g.far_rot), col0,
-                                  interior);
-      else
-        cp_async_commit();
-    }
-    cp_async_wait<NPF - 1>();
-    T f[NF][V];
+  // pass 0: the rows up to y1+1; pass 1 (le_step_soa's far end): rows ny-5 and ny-4 again
+  const int passes = FAR && !one_step && g.far_rot && y1 + 2 > g.ny ? 2 : 1;
+  for (int pass = 0; pass < passes && ok; ++pass) {
+    const int again = max(g.ny - 5, 0);
+    // rows marched, and step-A rows handed over (pass 0: see row_uses)
+    const int mbeg = !FAR || pass == 0 ? y0 - 4 : again - 2;
+    const int mend = !FAR || pass == 0 ? (one_step ? y1 + 2 : min(y1 + 4, g.ny + 2)) : (y1 == g.ny ? max(g.ny - 4, 0) : again) + 3;
+    ya.init();
 #pragma unroll
-    for (int k = 0; k < NF; ++k)
-      unpack(*reinterpret_cast<const VT*>(in_ring + islot * kRow + k * kIn), f[k]);
-    if (!interior) clamp_lane<T, V>(f, col0, g.nx);
-    sweep_x_lane<T, V, XPACK>(f, cx);
-    ring_left(ya, f, a_ring, aslot, cy);
-    const int ka = m - 2;  // step-A row completed now
-    if (m >= y0 && row_uses(ka, y0, y1, g.ny, one_step) > 0) {
-      T ga[NF][V];
-      ring_output(ya, ga, a_ring, aslot, cy);
-      if (!interior) clamp_columns<T, V>(ga, xs, col0, g.nx);
-      const int hs = (int)(u % kHand);
-      const unsigned use = u / kHand;
-      if (use > 0 && !mbar_wait(empty + hs, (use - 1) & 1, wait_ns, status)) {
-        ok = false;
-        break;
+    for (int k = 0; k < NF; ++k) *reinterpret_cast<VT*>(a_ring + 2 * kRow + k * kIn) = VT{};
+#pragma unroll
+    for (int j = 0; j < NPF - 1; ++j)
+      fetch_row<T, V, COHERENT>(in_ring + j * kRow, g, source_row(mbeg + j, g.ny, g.far_rot), col0,
+                                interior);
+    int islot = 0, aslot = 0;
+    for (int m = mbeg; m < mend; ++m) {
+      {
+        const int mm = m + NPF - 1;
+        const int ns = islot + NPF - 1 >= NPF ? islot - 1 : islot + NPF - 1;
+        if (mm < mend)
+          fetch_row<T, V, COHERENT>(in_ring + ns * kRow, g, source_row(mm, g.ny, g.far_rot), col0,
+                                    interior);
+        else
+          cp_async_commit();
       }
-      T* slot = hand + hs * kRow;
+      cp_async_wait<NPF - 1>();
+      T f[NF][V];
 #pragma unroll
-      for (int k = 0; k < NF; ++k) *reinterpret_cast<VT*>(slot + k * kIn) = pack(ga[k]);
-      mbar_arrive(full + hs);
-      ++u;
+      for (int k = 0; k < NF; ++k)
+        unpack(*reinterpret_cast<const VT*>(in_ring + islot * kRow + k * kIn), f[k]);
+      if (!interior) clamp_lane<T, V>(f, col0, g.nx);
+      sweep_x_lane<T, V, XPACK>(f, cx);
+      ring_left(ya, f, a_ring, aslot, cy);
+      const int ka = m - 2;  // step-A row completed now
+      // handed over once for pass 0's uses; in pass 1 once for every row past ny-1 it stands for
+      int hands = 0;
+      if (!FAR || pass == 0)
+        hands = m >= y0 && ka < g.ny && row_uses(ka, y0, y1, g.ny, one_step, FAR && g.far_rot) > 0;
+      else if (m >= mbeg + 4)
+        hands = y1 == g.ny && g.ny < 5 ? 2 : 1;
+      if (hands > 0) {
+        T ga[NF][V];
+        ring_output(ya, ga, a_ring, aslot, cy);
+        if (!interior) clamp_columns<T, V>(ga, xs, col0, g.nx);
+        for (int h = 0; h < hands; ++h) {
+          const int hs = (int)(u % kHand);
+          const unsigned use = u / kHand;
+          if (use > 0 && !mbar_wait(empty + hs, (use - 1) & 1, wait_ns, status)) {
+            ok = false;
+            break;
+          }
+          T* slot = hand + hs * kRow;
+#pragma unroll
+          for (int k = 0; k < NF; ++k) *reinterpret_cast<VT*>(slot + k * kIn) = pack(ga[k]);
+          mbar_arrive(full + hs);
+          ++u;
+        }
+        if (!ok) break;
+      }
+      ya.right(cy);
+      islot = islot + 1 == NPF ? 0 : islot + 1;
+      aslot = aslot == 2 ? 0 : aslot + 1;
     }
-    ya.right(cy);
-    islot = islot + 1 == NPF ? 0 : islot + 1;
-    aslot = aslot == 2 ? 0 : aslot + 1;
   }
   cp_async_wait<0>();  // nothing of this warp's in flight when it leaves (also after a break)
   return ok;
@@ -431,7 +456,7 @@ __device__ __forceinline__ bool pair_produce(const GridRef<T>& g, const Sweep<T>
 // producer.  A one_step tile's handed rows are step A's rows [y0, y1), written as they
 // are.  TAP: receiver rows -- tap_a of the rows after step A (taken from the handed rows),
 // tap_b of the rows after step B.  Returns false if a wait gave up.
-template <typename T, int V, int NPF, bool TAP, bool XPACK = true, typename CY = Sweep<T>>
+template <typename T, int V, int NPF, bool TAP, bool FAR, bool XPACK = true, typename CY = Sweep<T>>
 __device__ __forceinline__ bool pair_consume(const GridRef<T>& g, const Sweep<T>& cx, const CY& cy, int strip,
                                              int y0, int y1, T* smem_pair,
                                              unsigned long long* bars,
@@ -459,7 +484,7 @@ __device__ __forceinline__ bool pair_consume(const GridRef<T>& g, const Sweep<T>
   int bslot = 0;
   int bin = y0 - 2;  // step-B row index of the next row fed to step B
   for (int ka = y0 - 2; ka < y1 + 2; ++ka) {
-    const int reps = row_uses(ka, y0, y1, g.ny, one_step);
+    const int reps = row_uses(ka, y0, y1, g.ny, one_step, FAR && g.far_rot);
     if (reps == 0) continue;
     const int hs = (int)(u % kHand);
     if (!mbar_wait(full + hs, (u / kHand) & 1, wait_ns, status)) return false;

@@ -119,8 +119,9 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) fused_step_kernel(const Fus
 
 // Two-step tiles on warp pairs: W / 2 pairs per block, each with its own shared
 // memory and queue barriers.  The barriers are initialised before the block's barrier, so
-// both warps of a pair see them, and the pair leaves together (same tile).
-template <typename T, int V, int MINB, int NPF, int W, int F>
+// both warps of a pair see them, and the pair leaves together (same tile).  FAR: le_step_soa's
+// far end.
+template <typename T, int V, int MINB, int NPF, int W, int F, bool FAR>
 __global__ void __launch_bounds__(W * 32, MINB) fused_pair_kernel(const FusedParams<T> p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int kPairs = W / 2;
@@ -156,10 +157,10 @@ __global__ void __launch_bounds__(W * 32, MINB) fused_pair_kernel(const FusedPar
     }
   }
   if (producer)
-    march::pair_produce<T, V, NPF, false>(p.g, p.c.x, ycons(p), strip, y0, y1, smem, bars, p.pair.wait_ns,
+    march::pair_produce<T, V, NPF, false, FAR>(p.g, p.c.x, ycons(p), strip, y0, y1, smem, bars, p.pair.wait_ns,
                                           p.pair.status, u, false);
   else
-    march::pair_consume<T, V, NPF, false>(p.g, p.c.x, ycons(p), strip, y0, y1, smem, bars, p.pair.wait_ns,
+    march::pair_consume<T, V, NPF, false, FAR>(p.g, p.c.x, ycons(p), strip, y0, y1, smem, bars, p.pair.wait_ns,
                                           p.pair.status, u, false, no_tap, no_tap);
 }
 
@@ -211,9 +212,10 @@ struct VariantKernel {
   using C = VariantCfg<T, VAR>;
   static_assert(C::P == 1 || C::W == kWarps, "block size: warp pairs only");
   static_assert(C::P == 1 || C::D == 1 || C::F == 0, "lean loops: warp pairs and one-step tiles");
-  static void* fn() {
+  static void* fn(bool far = false) {
     if constexpr (C::P == 1)
-      return (void*)fused_pair_kernel<T, C::V, C::MINB, C::NPF, C::W, C::F>;
+      return far ? (void*)fused_pair_kernel<T, C::V, C::MINB, C::NPF, C::W, C::F, true>
+                 : (void*)fused_pair_kernel<T, C::V, C::MINB, C::NPF, C::W, C::F, false>;
     else
       return (void*)fused_step_kernel<T, C::V, C::MINB, C::NPF, C::D, C::F>;
   }
@@ -227,20 +229,21 @@ struct VariantKernel {
   static void prepare() {
     static unsigned long long done = 0;  // bit d: device d (devices 0..63)
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
-      cudaFuncSetAttribute(fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem());
-      return;
-    }
-    if (!(done & (1ull << dev))) {
-      cudaFuncSetAttribute(fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem());
-      done |= 1ull << dev;
-    }
+    const bool known = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64;
+    if (known && (done >> dev & 1)) return;
+    for (int far = 0; far < (C::P == 1 ? 2 : 1); ++far)
+      cudaFuncSetAttribute(fn(far != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem());
+    if (known) done |= 1ull << dev;
   }
   static void launch(const FusedPlan& pl, const FusedParams<T>& p, cudaStream_t s) {
-    if constexpr (C::P == 1)
-      fused_pair_kernel<T, C::V, C::MINB, C::NPF, C::W, C::F><<<pl.blocks, pl.threads, pl.smem, s>>>(p);
-    else
+    if constexpr (C::P == 1) {
+      if (p.g.far_rot)
+        fused_pair_kernel<T, C::V, C::MINB, C::NPF, C::W, C::F, true><<<pl.blocks, pl.threads, pl.smem, s>>>(p);
+      else
+        fused_pair_kernel<T, C::V, C::MINB, C::NPF, C::W, C::F, false><<<pl.blocks, pl.threads, pl.smem, s>>>(p);
+    } else {
       fused_step_kernel<T, C::V, C::MINB, C::NPF, C::D, C::F><<<pl.blocks, pl.threads, pl.smem, s>>>(p);
+    }
   }
 };
 
@@ -442,7 +445,8 @@ cudaError_t launch_fused_rows(const T* src, T* dst, int nx, int ny, long long pi
                               const StepConsts<T>& c, int far_rot, const FusedPlan& plan,
                               const PairCtl& pair, int seg_len, int nranges, const int* lo,
                               const int* hi, cudaStream_t s) {
-  if (plan.depth == 2 && far_rot) return cudaErrorInvalidValue;  // two steps assume clamped ends
+  // two steps on one warp assume clamped ends; warp pairs know le_step_soa's far end
+  if (plan.depth == 2 && far_rot && plan.warps_per_task != 2) return cudaErrorInvalidValue;
   if (plan.warps_per_task == 2 && pair.status == nullptr) return cudaErrorInvalidValue;
   if (nranges < 1 || nranges > 2 || seg_len < 1) return cudaErrorInvalidValue;
   FusedParams<T> p;
