@@ -1131,6 +1131,20 @@ int le2d_diagnostics(le_task* task, le2d_diag_t* out) {
 
 namespace {
 
+// Whether a buffer a caller hands to le2d_rows_out / le2d_rows_in is memory of the current
+// device, aligned to T, which one kernel copies; anything else a copy call takes (another
+// device's memory, page-locked host memory) goes through one.
+bool copied_by_kernel(const T* buf) {
+  cudaPointerAttributes a;
+  int dev = -1;
+  if ((uintptr_t)buf % sizeof(T) != 0 || cudaGetDevice(&dev) != cudaSuccess ||
+      cudaPointerGetAttributes(&a, buf) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == dev;
+}
+
 // Rows [row0, row0 + nrows) of the task's state <-> a caller's device buffer laid out
 // [field][row][nx], on the caller's stream `stream`, ordered with the task's stream both ways
 // (events), so a caller can hand the rows to a collective on its own stream.
@@ -1145,8 +1159,11 @@ int copy_rows(le_task* task, int row0, int nrows, T* dev_buf, void* stream, bool
   const cudaStream_t s = (cudaStream_t)stream;
   cudaError_t e = cudaEventRecord(d->ev[0], d->stream);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(s, d->ev[0], 0);
-  for (int k = 0; k < 5 && e == cudaSuccess; ++k) {
-    T* state = d->buf[d->cur] + k * d->plane + (long long)row0 * d->pitch;
+  T* first = d->buf[d->cur] + (long long)row0 * d->pitch;
+  const bool kernel = e == cudaSuccess && copied_by_kernel(dev_buf);
+  if (kernel) e = le2d::launch_copy_rows<T>(first, dev_buf, d->nx, nrows, d->pitch, d->plane, out, s);
+  for (int k = 0; k < 5 && e == cudaSuccess && !kernel; ++k) {
+    T* state = first + k * d->plane;
     T* flat = dev_buf + (size_t)k * nrows * d->nx;
     if (out)
       e = cudaMemcpy2DAsync(flat, sizeof(T) * d->nx, state, sizeof(T) * d->pitch, sizeof(T) * d->nx, nrows,

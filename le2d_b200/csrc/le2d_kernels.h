@@ -109,6 +109,12 @@ template <typename T>
 cudaError_t launch_unpack(const T* soa, T* raw, int nx, int ny, long long pitch,
                           long long plane, int aos, cudaStream_t s);
 
+// Rows of the state (soa: field 0 of the first row) to (out) or from a flat device buffer
+// [field][row][nx], both on the current device; `flat` aligned to T.
+template <typename T>
+cudaError_t launch_copy_rows(T* soa, T* flat, int nx, int nrows, long long pitch, long long plane, bool out,
+                             cudaStream_t s);
+
 // The VTK writer's scalar: |v| of every node as a big-endian float32, rows j outer
 // (out: nx*ny words), the same bytes as the host writer computes.
 template <typename T>
