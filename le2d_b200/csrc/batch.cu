@@ -32,9 +32,6 @@
 // step A's rows down to ny-7, within the tile above the last one: tiles are at least 8 rows.)
 // A producer may claim its next item while its consumer still finishes the last one: all
 // rows of that item are already in the queue, so the consumer finishes without it.
-// The x-sweep runs one invariant at a time (sweep_x_lane_diff), which at this kernel's
-// occupancy is faster than the packed form the single-solve kernels use; both give the
-// same bits.
 #include <type_traits>
 
 #include "march_pair.cuh"
@@ -161,7 +158,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB)
     const long long step_after = I.abs_step0 + r + 1;  // absolute step count after this step
     if (I.trace != nullptr && step_after % I.trace_every == 0)
       tap = march::RowTap<T>{I.trace + (step_after / I.trace_every - 1) * 2 * I.pitch, I.trace_row};
-    march::march_tile<T, V, kNpf, true, true, false>(g, load_step_consts(cslot, I.c), bt.strip, y0, y1, ring,
+    march::march_tile<T, V, kNpf, true, true>(g, load_step_consts(cslot, I.c), bt.strip, y0, y1, ring,
                                                      tap);
     __syncwarp();
     const int tile_id = I.tile_base + bt.seg * I.nstrips + bt.strip;
@@ -258,7 +255,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB)
       const int y0 = bt.seg * I.seg_len;
       const int y1 = min(y0 + I.seg_len, I.ny);
       const ItemConsts<T>& k = load_item_consts(kslot, I);
-      if (!march::pair_produce<T, V, kNpf, true, true, false>(g, k.x, k.y, bt.strip, y0, y1, smem, bars, wait_ns,
+      if (!march::pair_produce<T, V, kNpf, true, true>(g, k.x, k.y, bt.strip, y0, y1, smem, bars, wait_ns,
                                                         status, u, nadv == 1))
         break;
     }
@@ -291,7 +288,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB)
         tap_b = march::RowTap<T>{I.trace + ((before + 2) / I.trace_every - 1) * 2 * I.pitch, I.trace_row};
       const int tile_id = I.tile_base + bt.seg * I.nstrips + bt.strip;
       const ItemConsts<T>& k = load_item_consts(kslot, I);
-      if (!march::pair_consume<T, V, kNpf, true, true, false>(g, k.x, k.y, bt.strip, y0, y1, smem, bars, wait_ns,
+      if (!march::pair_consume<T, V, kNpf, true, true>(g, k.x, k.y, bt.strip, y0, y1, smem, bars, wait_ns,
                                                         status, u, nadv == 1, tap_a, tap_b))
         break;
       __syncwarp();  // the consumer wrote the tile's new state and publishes it

@@ -24,7 +24,7 @@
 // FP32: difference form.  The flux differences need only the face differences D:
 //   A_i = F_{i-1} - F_i = t_{i-1} - psi_i D_i,        t_i = (psi_i - 1) D_i
 //   B_i = G_{i+1} - G_i = c_i - psi'_{i+1} D_i,       c_i = D_i + psi'_i D_{i-1}
-// and D itself is formed from differences of the fields (face_differences), so the
+// and D itself is formed from differences of the fields, so the
 // update never subtracts two large invariants: in FP32 this keeps the relative
 // accuracy of small increments (e.g. residual velocities next to large static stresses)
 // that differencing the invariants loses.  The field update uses the invariant changes
@@ -93,15 +93,7 @@ __device__ __forceinline__ float tvd_eps<float>() { return 1e-6f; }  // TVD2_EPS
 template <>
 __device__ __forceinline__ double tvd_eps<double>() { return 1e-6; }
 
-// Slope ratio a / b.  FP32: hardware reciprocal (rcp.approx, <= 1 ulp) times a;
-// for b = +-0 it gives +-inf (a != 0) or NaN (a = 0) like the division does, and the
-// limiter maps those exactly as the reference (superbee(+-inf) = 2 / 0, superbee(NaN) = 2).
-__device__ __forceinline__ float ratio(float a, float b) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
-  return a * r;
-}
-// FP64: Newton-Raphson division.  The hardware reciprocal estimate y0 (relative error
+// Slope ratio a / b in FP64: Newton-Raphson division (FP32: march.cuh).  The hardware reciprocal estimate y0 (relative error
 // around 2^-23) is refined by one Newton step y = y0 + y0 (1 - b y0) (error about its
 // square, 2^-46), and the quotient q = a y by one correction with its FMA residual,
 // r = q + (a - b q) y (Markstein's final step), whose error is of the order of the square
@@ -137,15 +129,9 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 }
 __device__ __forceinline__ double max3(double a, double b, double c) { return fmax(a, fmax(b, c)); }
 
-// kc * superbee(r), superbee(r) = max(0, min(1, 2r), min(2, r))  (simple/le_core.c:38);
-// the reference's le_min/le_max give superbee(NaN) = max(0, 1, 2) = 2.  FP32:
-// max(sat(2r), min(2, r)), the same function with one min/max less -- sat clamps 2r to [0, 1] (so r <= 0 gives 0 from both
-// terms) and flushes NaN to 0, while min(2, NaN) = 2, keeping superbee(NaN) = 2.
-__device__ __forceinline__ float psi(float r, float kc) {
-  return kc * fmaxf(__saturatef(r + r), fminf(2.0f, r));
-}
-__device__ __forceinline__ float psi_ratio(float a, float b, float kc) { return psi(ratio(a, b), kc); }
-// FP64: kc * superbee(a / b), the limited slope ratio, without floating-point compares.
+// kc * superbee(a / b), the limited slope ratio, in FP64 without floating-point compares;
+// superbee(r) = max(0, min(1, 2r), min(2, r))  (simple/le_core.c:38), and the reference's
+// le_min/le_max give superbee(NaN) = max(0, 1, 2) = 2.
 // superbee(r) is one of 0, 2r, 1, r and 2, and which one follows from r's high word h alone,
 // because the breakpoints 0.5, 1 and 2 have zero low words (so, for r >= 0, r < 1 <=>
 // h < h(1), and so on).  Below 1, t = h + 2^20 (one more in the exponent field: 2r, r being a
@@ -218,18 +204,6 @@ __device__ __forceinline__ void increment(double& vx, double& vy, double& sxx, d
 }
 }  // namespace ex
 
-// Differences of the four moving invariants across a face, formed from the differences
-// of the fields that enter them (normal velocity vn, normal stress sn, tangential
-// velocity vt, shear stress sxy) rather than by differencing the invariants.
-template <typename T>
-__device__ __forceinline__ void face_differences(T dvn, T dsn, T dvt, T dsxy, const Sweep<T>& c,
-                                                 T& d1, T& d2, T& d3, T& d4) {
-  d1 = fma(-dsn, c.irhoc1, dvn);
-  d2 = fma(dsn, c.irhoc1, dvn);
-  d3 = fma(-dsxy, c.irhoc2, dvt);
-  d4 = fma(dsxy, c.irhoc2, dvt);
-}
-
 // Invariants of one node for a sweep along AXIS (0 = x, 1 = y).
 template <int AXIS, typename T>
 __device__ __forceinline__ void omega(T vx, T vy, T sxx, T sxy, T syy, const Sweep<T>& c, T& w1,
@@ -243,23 +217,6 @@ __device__ __forceinline__ void omega(T vx, T vy, T sxx, T sxy, T syy, const Swe
   w2 = vn + n00;
   w3 = vt - n01;
   w4 = vt + n01;
-}
-
-// Field update of one node from the flux differences of its four invariants:
-// a1 = F1_{i-1} - F1_i, b2 = G2_{i+1} - G2_i, a3, b4 likewise (inc_x / inc_y).
-template <int AXIS, typename T>
-__device__ __forceinline__ void apply_increment(T& vx, T& vy, T& sxx, T& sxy, T& syy, T a1, T b2,
-                                                T a3, T b4, const Sweep<T>& c) {
-  T& vn = AXIS == 0 ? vx : vy;
-  T& vt = AXIS == 0 ? vy : vx;
-  T& sn = AXIS == 0 ? sxx : syy;
-  T& so = AXIS == 0 ? syy : sxx;
-  const T p = b2 - a1;
-  vn = fma(c.hk1, a1 + b2, vn);
-  vt = fma(c.hk2, a3 + b4, vt);
-  sn = fma(c.hk1rc1, p, sn);
-  so = fma(c.hk1rc3, p, so);
-  sxy = fma(c.hk2rc2, b4 - a3, sxy);
 }
 
 }  // namespace le2d

@@ -213,69 +213,6 @@ __device__ __forceinline__ void sweep_x_lane_exact(double (&f)[NF][V], const Swe
                      dw[2][v], dw[3][v], c);
 }
 
-// FP32 x-sweep of the V nodes of this lane in the difference form, one invariant at a time
-// (row in registers, neighbours by shuffles).  Face e (0..V) lies between node e-1 and
-// node e of the lane; the neighbour lanes supply the fields of nodes -1 and V and the flux
-// terms of their edge nodes.
-template <typename T, int V>
-__device__ __forceinline__ void sweep_x_lane_diff(T (&f)[NF][V], const Sweep<T>& c) {
-  constexpr unsigned kAll = 0xffffffffu;
-  const T eps = tvd_eps<T>();
-  // fields entering the x-invariants: vn = vx, sn = sxx, vt = vy, and sxy
-  T lf[4], rf[4];
-  {
-    const int fk[4] = {VX, SXX, VY, SXY};
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      lf[q] = __shfl_up_sync(kAll, f[fk[q]][V - 1], 1);
-      rf[q] = __shfl_down_sync(kAll, f[fk[q]][0], 1);
-    }
-  }
-  T d[4][V + 1];
-#pragma unroll
-  for (int e = 0; e <= V; ++e) {
-    const T nvx = e < V ? f[VX][e] : rf[0], pvx = e > 0 ? f[VX][e - 1] : lf[0];
-    const T nsx = e < V ? f[SXX][e] : rf[1], psx = e > 0 ? f[SXX][e - 1] : lf[1];
-    const T nvy = e < V ? f[VY][e] : rf[2], pvy = e > 0 ? f[VY][e - 1] : lf[2];
-    const T nxy = e < V ? f[SXY][e] : rf[3], pxy = e > 0 ? f[SXY][e - 1] : lf[3];
-    face_differences(nvx - pvx, nsx - psx, nvy - pvy, nxy - pxy, c, d[0][e], d[1][e], d[2][e],
-                     d[3][e]);
-  }
-  T a[2][V], b[2][V];
-#pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    const T kc = q ? c.kc2 : c.kc1;
-    {  // right-moving invariant (w1 / w3)
-      const int k = 2 * q;
-      T ps[V], t[V];
-#pragma unroll
-      for (int v = 0; v < V; ++v) {
-        ps[v] = psi_ratio(d[k][v] + eps, d[k][v + 1] + eps, kc);
-        t[v] = fma(ps[v], d[k][v + 1], -d[k][v + 1]);
-      }
-      const T t_in = __shfl_up_sync(kAll, t[V - 1], 1);
-#pragma unroll
-      for (int v = 0; v < V; ++v) a[q][v] = fma(-ps[v], d[k][v + 1], v ? t[v - 1] : t_in);
-    }
-    {  // left-moving invariant (w2 / w4)
-      const int k = 2 * q + 1;
-      T ps[V], h[V];
-#pragma unroll
-      for (int v = 0; v < V; ++v) {
-        ps[v] = psi_ratio(eps - d[k][v + 1], eps - d[k][v], kc);
-        h[v] = fma(-ps[v], d[k][v], d[k][v]);
-      }
-      const T h_in = __shfl_down_sync(kAll, h[0], 1);
-#pragma unroll
-      for (int v = 0; v < V; ++v) b[q][v] = fma(ps[v], d[k][v], v < V - 1 ? h[v + 1] : h_in);
-    }
-  }
-#pragma unroll
-  for (int v = 0; v < V; ++v)
-    apply_increment<0>(f[VX][v], f[VY][v], f[SXX][v], f[SXY][v], f[SYY][v], a[0][v], b[0][v],
-                       a[1][v], b[1][v], c);
-}
-
 // Packed FP32 arithmetic (f32x2: two independent lanes of the same operation, each
 // rounded as its scalar form).
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
@@ -288,30 +225,34 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __
 // 330.7 with the negated operand (195.3 / 202.8 Gnu/s), the same bits.
 __device__ __forceinline__ float2 neg2(float2 a) { return f2(-a.x, -a.y); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return add2(a, neg2(b)); }
+// superbee(r) = max(0, min(1, 2r), min(2, r)) (simple/le_core.c:38; 2 for NaN) as
+// max(sat(2r), min(2, r)), the same function with one min/max less: sat clamps 2r to [0, 1] (so
+// r <= 0 gives 0 from both terms) and flushes NaN to 0, while min(2, NaN) = 2.
 __device__ __forceinline__ float2 superbee2(float2 r) {
   return f2(fmaxf(__saturatef(r.x + r.x), fminf(2.0f, r.x)),
             fmaxf(__saturatef(r.y + r.y), fminf(2.0f, r.y)));
 }
-__device__ __forceinline__ float2 ratio2(float2 a, float2 b) {
+// Slope ratios a / b: hardware reciprocal (rcp.approx, <= 1 ulp) times a; for b = +-0 it
+// gives +-inf (a != 0) or NaN (a = 0) like the division does, and the limiter maps those as
+// the reference does (superbee(+-inf) = 2 / 0, superbee(NaN) = 2).
+__device__ __forceinline__ float2 rcp2(float2 b) {
   float x, y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(x) : "f"(b.x));
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b.y));
-  return mul2(a, f2(x, y));
+  return f2(x, y);
 }
+__device__ __forceinline__ float2 ratio2(float2 a, float2 b) { return mul2(a, rcp2(b)); }
 
 // FP32 x-sweep of the V nodes of this lane in the difference form (row in registers,
 // neighbours by shuffles), on pairs of invariants: (w1, w3) move right and (w2, w4) left,
 // and the two of a pair go through the same operations with their own constants, so each
 // pair runs as packed f32x2 arithmetic -- the field differences of a face are formed as
-// (dvx, dvy) and (dsxx, dsxy), which give (D1, D3) and (D2, D4) in one packed FMA each.
-// Every element sees the operations of sweep_x_lane_diff in the same order, with the
-// right-moving pair keeping -t and -A as the packed y-pipeline does.  The two forms give the same bits: t, A, -t and -A are never -0 (an
-// exact zero of a rounded sum is +0, and psi >= 0), so where A = +0 the sums A + B and
-// B - A that enter the fields are B + 0 in both.  About 9 % fewer instructions per
-// node-update in the fused kernels; the batched kernel, at a different occupancy, runs
-// the scalar form faster.  Face e (0..V) lies between node e-1 and node e of the lane;
-// the neighbour lanes supply the fields of nodes -1 and V and the flux terms of their edge
-// nodes.
+// (dvx, dvy) and (dsxx, dsxy), which give (D1, D3) and (D2, D4) in one packed FMA each.  The
+// right-moving pair keeps -t and -A as the packed y-pipeline does.  About 9 % fewer
+// instructions per node-update than one invariant at a time; the batched kernel, which ran
+// that form while negations cost it instructions, 2 % faster (48 instances 41.4 / 40.4 ms).
+// Face e (0..V) lies between node e-1 and node e of the lane; the neighbour lanes supply the
+// fields of nodes -1 and V and the flux terms of their edge nodes.
 //
 // MASK: `em[e]` (0 or 1) multiplies the differences of face e, for lanes that hold columns at
 // or beyond the grid's ends (block tiles, tile.cuh): a face with a clamped column has two equal
@@ -377,7 +318,7 @@ __device__ __forceinline__ void sweep_x_lane_packed(float (&f)[NF][V], const Swe
     for (int v = 0; v < V; ++v) b[v] = fma2(ps[v], dl[v], v < V - 1 ? h[v + 1] : h_in);
   }
 #pragma unroll
-  for (int v = 0; v < V; ++v) {  // apply_increment<0>
+  for (int v = 0; v < V; ++v) {  // the field update
     const float2 sum = sub2(b[v], na[v]);  // (A1 + B2, A3 + B4)
     const float2 dif = add2(b[v], na[v]);      // (B2 - A1, B4 - A3)
     f[VX][v] = fmaf(c.hk1, sum.x, f[VX][v]);
@@ -388,16 +329,14 @@ __device__ __forceinline__ void sweep_x_lane_packed(float (&f)[NF][V], const Swe
   }
 }
 
-// x-sweep of one lane's V nodes: FP32 in the difference form (invariant pairs packed when
-// XPACK), FP64 in the reference's flux form.
-template <typename T, int V, bool XPACK = true>
+// x-sweep of one lane's V nodes: FP32 in the difference form, FP64 in the reference's flux
+// form.
+template <typename T, int V>
 __device__ __forceinline__ void sweep_x_lane(T (&f)[NF][V], const Sweep<T>& c) {
   if constexpr (sizeof(T) == 8)
     sweep_x_lane_exact<V>(f, c);
-  else if constexpr (XPACK)
-    sweep_x_lane_packed<V>(f, c);
   else
-    sweep_x_lane_diff<T, V>(f, c);
+    sweep_x_lane_packed<V>(f, c);
 }
 
 // Shared memory of one warp: NPF rows of raw input (filled by cp.async, NPF-1 rows ahead)
@@ -586,21 +525,23 @@ struct YPipe<double, V> {
 };
 
 // FP32: the same pipeline on pairs of columns with packed f32x2 arithmetic (the columns
-// are independent in the y-sweep).  The right-moving state keeps -t and -A.  Reciprocals and the limiter's min/max/sat stay
+// are independent in the y-sweep).  The right-moving state keeps -t and -A; the left-moving
+// one the reciprocal of Q_{m-2}, taken where Q was formed, into the register it stays in (Q
+// itself would have to be copied each row: 8192^2 324.5 / 323.6 us a step).  Reciprocals and the limiter's min/max/sat stay
 // per element.
 
 template <int V>
 struct YPipe<float, V> {
   static_assert(V % 2 == 0, "pairs of columns");
   static constexpr int P = V / 2;
-  float2 p2[2][P], nt2[2][P], na2[2][P], q2[2][P], d2[2][P], c2[2][P];
+  float2 p2[2][P], nt2[2][P], na2[2][P], rq2[2][P], d2[2][P], c2[2][P];
   float2 dfw[2][P], bo[2][P];
 
   __device__ __forceinline__ void init() {
 #pragma unroll
     for (int i = 0; i < P; ++i)
 #pragma unroll
-      for (int q = 0; q < 2; ++q) p2[q][i] = nt2[q][i] = na2[q][i] = q2[q][i] = d2[q][i] = c2[q][i] = f2(0.f, 0.f);
+      for (int q = 0; q < 2; ++q) p2[q][i] = nt2[q][i] = na2[q][i] = rq2[q][i] = d2[q][i] = c2[q][i] = f2(0.f, 0.f);
   }
 
   // The constants come as pairs (YPairs); the Sweep overloads pair them up in registers.
@@ -622,12 +563,12 @@ struct YPipe<float, V> {
         dfw[q][i] = d[2 * q];
         const float2 dd = d[2 * q + 1];
         const float2 q1 = sub2(eps, dd);
-        const float2 phi = superbee2(ratio2(q1, q2[q][i]));
+        const float2 phi = superbee2(mul2(q1, rq2[q][i]));
         const float2 ps = mul2(q ? yc.k2 : yc.k1, phi);
         bo[q][i] = fma2(neg2(ps), d2[q][i], c2[q][i]);  // c - psi' D_{m-2}
         c2[q][i] = fma2(ps, d2[q][i], dd);         // D + psi' D_{m-2}
         d2[q][i] = dd;
-        q2[q][i] = q1;
+        rq2[q][i] = rcp2(q1);
       }
     }
   }
@@ -681,9 +622,9 @@ struct YPipe<float, V> {
 };
 
 // Advances one tile -- strip `strip` (32*V columns, halo lanes included), rows [y0, y1) --
-// by one step from g.src to g.dst (XPACK: the x-sweep's form, see sweep_x_lane).  `smem_warp` = this warp's warp_smem_elems() elements of
+// by one step from g.src to g.dst.  `smem_warp` = this warp's warp_smem_elems() elements of
 // shared memory; every lane touches only its own V columns of it.  Called by all 32 lanes.
-template <typename T, int V, int NPF, bool COHERENT, bool TAP, bool XPACK = true>
+template <typename T, int V, int NPF, bool COHERENT, bool TAP>
 __device__ __forceinline__ void march_tile(const GridRef<T>& g, const StepConsts<T>& c, int strip,
                                            int y0, int y1, T* smem_warp, const RowTap<T>& tap) {
   using VT = typename Vec<T, V>::type;
@@ -733,7 +674,7 @@ __device__ __forceinline__ void march_tile(const GridRef<T>& g, const StepConsts
       unpack(*reinterpret_cast<const VT*>(in_ring + islot * kRow + k * kIn), f[k]);
     if (!interior) clamp_lane<T, V>(f, col0, g.nx);
 
-    sweep_x_lane<T, V, XPACK>(f, c.x);
+    sweep_x_lane<T, V>(f, c.x);
 
     T* rs = xs_ring + xslot * kRow;
 #pragma unroll

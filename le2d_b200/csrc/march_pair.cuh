@@ -359,7 +359,7 @@ __device__ __forceinline__ void march_tile_interior(const GridRef<T>& g, const S
 // the consumer; `u` counts the queue's handoffs (it continues across tiles).  A one_step
 // tile (an odd last step) hands over step A's rows [y0, y1) only, which the consumer writes.
 // Returns false if a wait gave up.
-template <typename T, int V, int NPF, bool COHERENT, bool FAR, bool XPACK = true, typename CY = Sweep<T>>
+template <typename T, int V, int NPF, bool COHERENT, bool FAR, typename CY = Sweep<T>>
 __device__ __forceinline__ bool pair_produce(const GridRef<T>& g, const Sweep<T>& cx, const CY& cy, int strip,
                                              int y0, int y1, T* smem_pair,
                                              unsigned long long* bars,
@@ -415,7 +415,7 @@ __device__ __forceinline__ bool pair_produce(const GridRef<T>& g, const Sweep<T>
       for (int k = 0; k < NF; ++k)
         unpack(*reinterpret_cast<const VT*>(in_ring + islot * kRow + k * kIn), f[k]);
       if (!interior) clamp_lane<T, V>(f, col0, g.nx);
-      sweep_x_lane<T, V, XPACK>(f, cx);
+      sweep_x_lane<T, V>(f, cx);
       ring_left(ya, f, a_ring, aslot, cy);
       const int ka = m - 2;  // step-A row completed now
       // handed over once for pass 0's uses; in pass 1 once for every row past ny-1 it stands for
@@ -456,7 +456,7 @@ __device__ __forceinline__ bool pair_produce(const GridRef<T>& g, const Sweep<T>
 // producer.  A one_step tile's handed rows are step A's rows [y0, y1), written as they
 // are.  TAP: receiver rows -- tap_a of the rows after step A (taken from the handed rows),
 // tap_b of the rows after step B.  Returns false if a wait gave up.
-template <typename T, int V, int NPF, bool TAP, bool FAR, bool XPACK = true, typename CY = Sweep<T>>
+template <typename T, int V, int NPF, bool TAP, bool FAR, typename CY = Sweep<T>>
 __device__ __forceinline__ bool pair_consume(const GridRef<T>& g, const Sweep<T>& cx, const CY& cy, int strip,
                                              int y0, int y1, T* smem_pair,
                                              unsigned long long* bars,
@@ -511,7 +511,7 @@ __device__ __forceinline__ bool pair_consume(const GridRef<T>& g, const Sweep<T>
 #pragma unroll
       for (int k = 0; k < NF; ++k) unpack(*reinterpret_cast<const VT*>(slot + k * kIn), fb[k]);
       if (r == reps - 1) mbar_arrive(empty + hs);
-      sweep_x_lane<T, V, XPACK>(fb, cx);
+      sweep_x_lane<T, V>(fb, cx);
       ring_left(yb, fb, b_ring, bslot, cy);
       if (bin >= y0 + 2) {  // step-B row bin-2 is complete
         T gb[NF][V];
