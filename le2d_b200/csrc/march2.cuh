@@ -52,15 +52,11 @@ __device__ __forceinline__ void clamp_columns(T (&v)[NF][V], int xs, int col0, i
 // row back (aligned loads), advance the left-moving part.  `cy`: the y-sweep constants
 // (Sweep, or YPairs for the FP32 pipeline).
 template <typename T, int V, typename CY>
-__device__ __forceinline__ void ring_left(YPipe<T, V>& yp, T (&f)[NF][V], T* ring, int slot,
-                                          const CY& cy) {
+__device__ __forceinline__ void rows_left(YPipe<T, V>& yp, T (&f)[NF][V], T* rs, const T* rp, const CY& cy) {
   using VT = typename Vec<T, V>::type;
   constexpr int kIn = 32 * V;
-  constexpr int kRow = NF * kIn;
-  T* rs = ring + slot * kRow;
 #pragma unroll
   for (int k = 0; k < NF; ++k) *reinterpret_cast<VT*>(rs + k * kIn) = pack(f[k]);
-  const T* rp = ring + (slot == 0 ? 2 : slot - 1) * kRow;
   T cur[NF][V], pvy[V], psyy[V], pvx[V], psxy[V];
   unpack(*reinterpret_cast<const VT*>(rs + VY * kIn), cur[VY]);
   unpack(*reinterpret_cast<const VT*>(rs + SYY * kIn), cur[SYY]);
@@ -72,19 +68,44 @@ __device__ __forceinline__ void ring_left(YPipe<T, V>& yp, T (&f)[NF][V], T* rin
   unpack(*reinterpret_cast<const VT*>(rp + SXY * kIn), psxy);
   yp.left(cur, pvy, psyy, pvx, psxy, cy);
 }
+template <typename T, int V, typename CY>
+__device__ __forceinline__ void ring_left(YPipe<T, V>& yp, T (&f)[NF][V], T* ring, int slot,
+                                          const CY& cy) {
+  constexpr int kRow = NF * 32 * V;
+  rows_left(yp, f, ring + slot * kRow, ring + (slot == 0 ? 2 : slot - 1) * kRow, cy);
+}
 
 // The row two above, completed: fields from the ring plus the pipeline's increments.
 template <typename T, int V, typename CY>
-__device__ __forceinline__ void ring_output(const YPipe<T, V>& yp, T (&out)[NF][V], const T* ring,
-                                            int slot, const CY& cy) {
+__device__ __forceinline__ void row_output(const YPipe<T, V>& yp, T (&out)[NF][V], const T* rg, const CY& cy) {
   using VT = typename Vec<T, V>::type;
   constexpr int kIn = 32 * V;
-  constexpr int kRow = NF * kIn;
-  const T* rg = ring + (slot == 2 ? 0 : slot + 1) * kRow;
 #pragma unroll
   for (int k = 0; k < NF; ++k) unpack(*reinterpret_cast<const VT*>(rg + k * kIn), out[k]);
   yp.apply(out, cy);
 }
+template <typename T, int V, typename CY>
+__device__ __forceinline__ void ring_output(const YPipe<T, V>& yp, T (&out)[NF][V], const T* ring,
+                                            int slot, const CY& cy) {
+  constexpr int kRow = NF * 32 * V;
+  row_output(yp, out, ring + (slot == 2 ? 0 : slot + 1) * kRow, cy);
+}
+
+// The three rows of a ring as the pairs' lean loops hold them: rows m, m-1 and m-2, turned by one
+// after every row instead of found from a slot number (132.7 -> 130.3 instructions per
+// node-update; 8192^2 323.4 -> 319.9, 4096^2 89.4 -> 87.9 us a step).  The FP64 one-step loop, at
+// its 128 registers, lost 3 % by it.
+template <typename T>
+struct RingRows {
+  T *cur, *prev, *prev2;
+  __device__ __forceinline__ RingRows(T* ring, int row) : cur(ring), prev(ring + 2 * row), prev2(ring + row) {}
+  __device__ __forceinline__ void turn() {
+    T* t = prev2;
+    prev2 = prev;
+    prev = cur;
+    cur = t;
+  }
+};
 
 // Advances one tile -- strip `strip`, rows [y0, y1) -- by two steps from g.src to g.dst.
 // `smem_warp` = this warp's warp_smem_elems2() elements.  Called by all 32 lanes.

@@ -209,7 +209,7 @@ __device__ __forceinline__ bool pair_produce_interior(const GridRef<T>& g, const
     LE2D_FETCH_INTERIOR(T, V, in_ring + j * kRow, next, g);
     next += g.pitch;
   }
-  int aslot = 0;
+  RingRows<T> ring(a_ring, kRow);
   int islot = 0;  // input slot of row m; row m+NPF-1 goes to the slot before it
   bool ok = true;
   for (int m = y0 - 4; m < mend; ++m) {
@@ -224,13 +224,12 @@ __device__ __forceinline__ bool pair_produce_interior(const GridRef<T>& g, const
 #pragma unroll
     for (int k = 0; k < NF; ++k) unpack(*reinterpret_cast<const VT*>(in_ring + islot * kRow + k * kIn), f[k]);
     sweep_x_lane<T, V>(f, cx);
-    ring_left(ya, f, a_ring, aslot, cy);
+    rows_left(ya, f, ring.cur, ring.prev, cy);
     if (m >= y0) {  // step-A row m-2 is complete and handed over
       T ga[NF][V];
-      ring_output(ya, ga, a_ring, aslot, cy);
+      row_output(ya, ga, ring.prev2, cy);
       const int hs = (int)(u % kHand);
-      const unsigned use = u / kHand;
-      if (use > 0 && !mbar_wait(empty + hs, (use - 1) & 1, wait_ns, status)) {
+      if (!mbar_wait(empty + hs, (u / kHand - 1) & 1, wait_ns, status)) {  // at once for the first use
         ok = false;
         break;
       }
@@ -242,7 +241,7 @@ __device__ __forceinline__ bool pair_produce_interior(const GridRef<T>& g, const
     }
     ya.right(cy);
     islot = islot + 1 == NPF ? 0 : islot + 1;
-    aslot = aslot == 2 ? 0 : aslot + 1;
+    ring.turn();
   }
   cp_async_wait<0>();  // nothing of this warp's in flight when it leaves (also after a break)
   return ok;
@@ -270,7 +269,7 @@ __device__ __forceinline__ bool pair_consume_interior(const GridRef<T>& g, const
 #pragma unroll
   for (int k = 0; k < NF; ++k) *reinterpret_cast<VT*>(b_ring + 2 * kRow + k * kIn) = VT{};
   T* out = g.dst + (long long)y0 * g.pitch + xs + lane * V;  // next row written
-  int bslot = 0;
+  RingRows<T> ring(b_ring, kRow);
   for (int ka = y0 - 2; ka < y1 + 2; ++ka) {
     const int hs = (int)(u % kHand);
     if (!mbar_wait(full + hs, (u / kHand) & 1, wait_ns, status)) return false;
@@ -280,16 +279,16 @@ __device__ __forceinline__ bool pair_consume_interior(const GridRef<T>& g, const
     for (int k = 0; k < NF; ++k) unpack(*reinterpret_cast<const VT*>(slot + k * kIn), fb[k]);
     mbar_arrive(empty + hs);
     sweep_x_lane<T, V>(fb, cx);
-    ring_left(yb, fb, b_ring, bslot, cy);
+    rows_left(yb, fb, ring.cur, ring.prev, cy);
     if (ka >= y0 + 2) {  // step-B row ka-2 is complete
       T gb[NF][V];
-      ring_output(yb, gb, b_ring, bslot, cy);
+      row_output(yb, gb, ring.prev2, cy);
 #pragma unroll
       for (int k = 0; k < NF; ++k) store_if(writer && in_dst(g, out + k * g.plane, V), reinterpret_cast<VT*>(out + k * g.plane), pack(gb[k]));
       out += g.pitch;
     }
     yb.right(cy);
-    bslot = bslot == 2 ? 0 : bslot + 1;
+    ring.turn();
     ++u;
   }
   return true;

@@ -171,6 +171,8 @@ __global__ void __launch_bounds__(W * 32, MINB) fused_pair_kernel(const FusedPar
 // warps per block W, and F: 1 = interior tiles on the lean loops, 2 = the same with the
 // boundary tiles dealt out first (boundary_first: the general loops they take run beside
 // the lean ones on an SM only at the start of the launch, which ends on lean tiles).
+// Variant 13's input ring holds three rows, two in flight: 8192^2 319.9 / 316.8, 4096^2 87.9 / 87.3
+// us a step with two and three (eight pairs per SM fit either way).
 template <typename T, int VAR>
 struct VariantCfg;
 template <> struct VariantCfg<float, 0> { static constexpr int V = 4, MINB = 3, NPF = 2, D = 1, P = 0, W = 4, F = 0; };
@@ -186,7 +188,7 @@ template <> struct VariantCfg<float, 9> { static constexpr int V = 4, MINB = 4, 
 template <> struct VariantCfg<float, 10> { static constexpr int V = 4, MINB = 3, NPF = 3, D = 2, P = 1, W = 4, F = 0; };
 template <> struct VariantCfg<float, 11> { static constexpr int V = 4, MINB = 4, NPF = 2, D = 2, P = 1, W = 4, F = 1; };
 template <> struct VariantCfg<float, 12> { static constexpr int V = 4, MINB = 8, NPF = 2, D = 2, P = 1, W = 2, F = 1; };
-template <> struct VariantCfg<float, 13> { static constexpr int V = 4, MINB = 8, NPF = 2, D = 2, P = 1, W = 2, F = 2; };
+template <> struct VariantCfg<float, 13> { static constexpr int V = 4, MINB = 8, NPF = 3, D = 2, P = 1, W = 2, F = 2; };
 template <> struct VariantCfg<float, 14> { static constexpr int V = 4, MINB = 4, NPF = 2, D = 1, P = 0, W = 4, F = 2; };
 template <> struct VariantCfg<float, 15> { static constexpr int V = 4, MINB = 5, NPF = 2, D = 1, P = 0, W = 4, F = 2; };
 template <> struct VariantCfg<double, 0> { static constexpr int V = 2, MINB = 2, NPF = 2, D = 1, P = 0, W = 4, F = 0; };
