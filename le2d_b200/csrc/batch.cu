@@ -35,6 +35,7 @@
 #include <type_traits>
 
 #include "march_pair.cuh"
+#include "tile.cuh"
 
 namespace le2d {
 
@@ -300,6 +301,84 @@ __global__ void __launch_bounds__(kWarps * 32, MINB)
   }
 }
 
+// ---- block tiles ----
+
+// Windows whose time is the chain of dependent items rather than the work (few or small
+// instances) run on block tiles (tile.cuh) instead: a block claims an item, waits for its
+// dependencies as above and advances the tile by up to `depth` steps in registers.  A strip's
+// item takes 18 us for two steps at the least (20 rows march one after another), a block
+// tile's 4 us and 2 us a step.  Receiver lines are recorded from the registers after the step
+// they belong to.
+template <typename T>
+struct BatchShape;
+template <> struct BatchShape<float> { static constexpr int V = 2, R = 4, W = 12, D = 6; };
+template <> struct BatchShape<double> { static constexpr int V = 2, R = 2, W = 12, D = 3; };
+
+template <typename T>
+struct TileConsts {
+  Sweep<T> x;
+  typename std::conditional<sizeof(T) == 4, YPairs, Sweep<T>>::type y;
+};
+__device__ __forceinline__ const YPairs& item_ycons(const BatchInst<float>& I) { return I.yq; }
+__device__ __forceinline__ const Sweep<double>& item_ycons(const BatchInst<double>& I) { return I.c.y; }
+
+template <typename T, int V, int R, int W>
+__global__ void __launch_bounds__(W * 32, 1)
+    batch_tile_kernel(const BatchInst<T>* __restrict__ insts, const BatchTile* __restrict__ tiles,
+                      const long long* __restrict__ step_items, int nsteps, int depth, int* done, BatchCtl* ctl,
+                      unsigned long long wait_ns, int stall_plus1) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ long long s_item;
+  __shared__ int s_ok;
+  __shared__ TileConsts<T> s_c;
+  const long long total = step_items[nsteps];
+  int r = 0;
+  while (true) {
+    if (threadIdx.x == 0) s_item = (long long)atomicAdd(&ctl->next, 1ULL);
+    __syncthreads();
+    const long long q = s_item;
+    if (q >= total) break;
+    while (q >= step_items[r + 1]) ++r;
+    const BatchTile bt = tiles[q - step_items[r]];
+    const BatchInst<T>& I = insts[bt.inst];
+    if (threadIdx.x < 32) {
+      const bool ok = item_ready(I, bt, r, done, ctl, wait_ns);
+      if (threadIdx.x == 0) s_ok = ok ? 1 : launch_ending(ctl) ? -1 : 0;
+    } else {  // the item's constants meanwhile
+      constexpr int kx = (int)(sizeof(Sweep<T>) / 4), ky = (int)(sizeof(s_c.y) / 4);
+      const unsigned* sx = reinterpret_cast<const unsigned*>(&I.c.x);
+      const unsigned* sy = reinterpret_cast<const unsigned*>(&item_ycons(I));
+      for (int i = threadIdx.x - 32; i < kx; i += W * 32 - 32) reinterpret_cast<unsigned*>(&s_c.x)[i] = sx[i];
+      for (int i = threadIdx.x - 32; i < ky; i += W * 32 - 32) reinterpret_cast<unsigned*>(&s_c.y)[i] = sy[i];
+    }
+    __syncthreads();
+    const int ok = s_ok;
+    if (ok <= 0) {  // the instance failed: skip the item
+      if (ok < 0) break;
+      continue;
+    }
+    const int nadv = min(depth, I.steps - r * depth);
+    const int par = (I.parity + r) & 1;
+    const march::GridRef<T> g{I.buf[par], I.buf[par ^ 1], I.nx, I.ny, I.pitch, I.plane, I.far_rot};
+    const int ox0 = bt.strip * I.out_x, ox1 = min(ox0 + I.out_x, I.nx);
+    const int oy0 = (int)((long long)bt.seg * I.ny / I.nsegs), oy1 = (int)((long long)(bt.seg + 1) * I.ny / I.nsegs);
+    march::BlockTap<T> tap{nullptr, -1, 1, 1};
+    if (I.trace != nullptr) {
+      const long long before = I.abs_step0 + (long long)r * depth, samples = before / I.trace_every;
+      tap = march::BlockTap<T>{I.trace + samples * 2 * I.pitch, I.trace_row, I.trace_every,
+                               (int)((samples + 1) * I.trace_every - before)};
+    }
+    march::block_tile<T, V, R, W, true, true>(g, s_c.x, s_c.y, ox0, ox1, oy0, oy1, depth, nadv,
+                                              reinterpret_cast<T*>(smem_raw), tap);
+    __syncthreads();  // the tile's new state is written, its constants read
+    const int tile_id = I.tile_base + bt.seg * I.nstrips + bt.strip;
+    if (threadIdx.x == 0 && !(r == 0 && tile_id == stall_plus1 - 1)) {
+      __threadfence();
+      st_release(done + tile_id, r + 1);
+    }
+  }
+}
+
 template <typename T>
 struct BatchKernelOf;
 // FP32: two-step items on warp pairs (4 columns per lane, 168 registers: 12 warps per SM);
@@ -366,6 +445,40 @@ cudaError_t launch_batch(const BatchInst<T>* insts, const BatchTile* tiles,
   return cudaGetLastError();
 }
 
+template <typename T>
+BatchTileShape batch_tile_shape() {
+  using S = BatchShape<T>;
+  // a and b from batches of two 100 x 100 instances at 1 to D steps per item
+  constexpr bool f32 = sizeof(T) == 4;
+  return BatchTileShape{32 * S::V, S::R * S::W, S::D, f32 ? 4.1 : 4.9, f32 ? 2.1 : 3.5, f32 ? 1.2 : 1.15};
+}
+
+template <typename T>
+int batch_tile_resident_blocks(int device) {
+  using S = BatchShape<T>;
+  const void* fn = (const void*)batch_tile_kernel<T, S::V, S::R, S::W>;
+  constexpr size_t smem = march::block_tile_smem<T, S::V, S::R, S::W>();
+  int sms = 0, per_sm = 0;
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, S::W * 32, smem) != cudaSuccess) return 0;
+  return sms * per_sm;
+}
+
+template <typename T>
+cudaError_t launch_batch_tiles(const BatchInst<T>* insts, const BatchTile* tiles, const long long* step_items,
+                               int nsteps, long long total_items, int depth, int* done, BatchCtl* ctl,
+                               unsigned long long wait_ns, int stall_plus1, int resident_blocks, cudaStream_t s) {
+  using S = BatchShape<T>;
+  if (depth < 1 || depth > S::D) return cudaErrorInvalidValue;
+  long long blocks = total_items < resident_blocks ? total_items : resident_blocks;  // persistent: all resident
+  if (blocks < 1) blocks = 1;
+  batch_tile_kernel<T, S::V, S::R, S::W>
+      <<<(int)blocks, S::W * 32, march::block_tile_smem<T, S::V, S::R, S::W>(), s>>>(
+          insts, tiles, step_items, nsteps, depth, done, ctl, wait_ns, stall_plus1);
+  return cudaGetLastError();
+}
+
 #ifdef LE2D_CHECK
 unsigned long long check_violations_batch() {
   unsigned long long v = 0, zero = 0;
@@ -385,7 +498,13 @@ unsigned long long check_violations_batch() {
   template int batch_resident_blocks<T>(int);                                                   \
   template cudaError_t launch_batch<T>(const BatchInst<T>*, const BatchTile*, const long long*, \
                                        int, long long, int*, BatchCtl*, unsigned long long, int, \
-                                       int, cudaStream_t);
+                                       int, cudaStream_t);                                      \
+  template BatchTileShape batch_tile_shape<T>();                                                \
+  template int batch_tile_resident_blocks<T>(int);                                              \
+  template cudaError_t launch_batch_tiles<T>(const BatchInst<T>*, const BatchTile*,             \
+                                             const long long*, int, long long, int, int*,       \
+                                             BatchCtl*, unsigned long long, int, int,           \
+                                             cudaStream_t);
 LE2D_INST(float)
 LE2D_INST(double)
 #undef LE2D_INST

@@ -100,10 +100,17 @@ Engine<T>::Engine(size_t budget) {
   int dev = 0;
   cudaGetDevice(&dev);
   resident_blocks_ = batch_resident_blocks<T>(dev);
+  tile_blocks_ = batch_tile_resident_blocks<T>(dev);
   // Test hook for the bounded-wait path: in the engine's first window, tile k of the work
   // list never publishes its first step, so its instance fails (LE2D_ETIMEOUT) while the
   // other instances finish.
-  if (const char* s = getenv("LE2D_TEST_STALL_TILE")) stall_tile_ = atoi(s);
+  // LE2D_TEST_STALL_TILE stalls a strip's tile (windows then run on strips), LE2D_TEST_STALL_BLOCK
+  // tile k of whatever the window runs on.
+  if (const char* s = getenv("LE2D_TEST_STALL_TILE")) {
+    stall_tile_ = atoi(s);
+    stall_strips_ = true;
+  }
+  if (const char* s = getenv("LE2D_TEST_STALL_BLOCK")) stall_tile_ = atoi(s);
 }
 
 template <typename T>
@@ -386,9 +393,9 @@ int Engine<T>::read_failures(const std::vector<int>& ids) {
   return LE2D_OK;
 }
 
-// Tall tiles march fewer halo and pipeline-fill rows; short ones shorten the chain of dependent
-// items a small instance's steps are.  The height L with the least model of the window's time,
-// the larger of
+// Strips.  Tall tiles march fewer halo and pipeline-fill rows; short ones shorten the chain of
+// dependent items a small instance's steps are.  The height L with the least model of the
+// window's time, the larger of
 //   work:  sum over the instances of items x tiles(L) x (L + h) rows, shared by the resident
 //          tile slots, at the loaded time per row, and
 //   chain: the most items of an instance x (L + g) rows at the unloaded time per row
@@ -397,26 +404,55 @@ int Engine<T>::read_failures(const std::vector<int>& ids) {
 // 0.95 us; FP64 h = 5.3, 1.49 us, g = 18, 1.05 us.  Measured (ms, 64 rows as before / the
 // height picked): FP32 48 instances 44.9 / 42.8, 24 instances 20.8 / 10.1; FP64 112.8 / 110.9
 // and 43.2 / 23.4; the 24 as requests at a server 29.4 / 16.3 and 59.7 / 36.
+// Block tiles.  The same two sums over an item's time a + b d for d steps, every SM one tile at
+// a time, a little slower where all of them are busy; taken where they are less.  Measured (ms,
+// strips / block tiles at the depth picked): 8 instances with sides of 64 to 300 and 100 to 300
+// steps FP32 2.94 / 0.92, FP64 5.18 / 2.22; 32 of them 3.60 / 2.55 and 6.50 / 8.01 (strips kept);
+// the 24 above FP32 9.3 / 11.3 all on tiles, 8.5 with each window cut as it is faster.
 template <typename T>
-int Engine<T>::window_rows(const std::vector<std::pair<int, int>>& order) const {
+typename Engine<T>::Cut Engine<T>::cut_window(const std::vector<std::pair<int, int>>& steps) const {
   constexpr bool f32 = sizeof(T) == 4;
   constexpr double h = f32 ? 7.0 : 5.3, loaded = f32 ? 1.64 : 1.49, g = f32 ? 34.0 : 18.0, alone = f32 ? 0.95 : 1.05;
   const double slots = std::max(1, resident_blocks_) * (double)batch_block_items<T>();
+  const auto join = [](double work, double chain) {
+    return std::pow(std::pow(work, 8.0) + std::pow(chain, 8.0), 0.125);
+  };
   constexpr int heights[] = {8, 12, 16, 24, 32, 48, 64};
-  int best = heights[0];
+  Cut best;
   double least = 1e300;
+  bool own = depth_set_ != 0 || stall_strips_;  // tile heights or depths of the instances' own: strips
   for (int rows : heights) {
     double work = 0.0, chain = 0.0;
-    for (const auto& o : order) {
+    for (const auto& o : steps) {
       const Inst& in = insts_[o.second];
+      own = own || in.seg_len != 0;
       const int l = std::min(in.seg_len ? in.seg_len : rows, in.p.ny);
-      work += (double)o.first * in.nstrips * ((in.p.ny + l - 1) / l) * (l + h);
-      chain = std::max(chain, o.first * (l + g));
+      const int items = (o.first + in.depth - 1) / in.depth;
+      work += (double)items * in.nstrips * ((in.p.ny + l - 1) / l) * (l + h);
+      chain = std::max(chain, items * (l + g));
     }
-    const double t = std::pow(std::pow(work / slots * loaded, 8.0) + std::pow(chain * alone, 8.0), 0.125);
+    const double t = join(work / slots * loaded, chain * alone);
     if (t < least) {
       least = t;
-      best = rows;
+      best.rows = rows;
+    }
+  }
+  if (own || tile_blocks_ < 1) return best;
+  const BatchTileShape shape = batch_tile_shape<T>();
+  for (int d = 1; d <= shape.max_depth; ++d) {
+    double work = 0.0, chain = 0.0;
+    const int ox = shape.cols - 4 * d, oy = shape.rows - 4 * d;
+    for (const auto& o : steps) {
+      const Inst& in = insts_[o.second];
+      const int items = (o.first + d - 1) / d;
+      const double item = shape.a + shape.b * d;
+      work += items * item * ((in.p.nx + ox - 1) / ox) * ((in.p.ny + oy - 1) / oy);
+      chain = std::max(chain, items * item);
+    }
+    const double t = join(work / tile_blocks_ * shape.loaded, chain);
+    if (t < least) {
+      least = t;
+      best.tile_depth = d;
     }
   }
   return best;
@@ -434,18 +470,27 @@ typename Engine<T>::Window Engine<T>::plan_window(int window, const std::vector<
     const long long left = in.p.steps - done[id];
     if (left <= 0) continue;
     steps_of[id] = (int)std::min<long long>(left, window);
-    order.push_back({(steps_of[id] + in.depth - 1) / in.depth, id});
+    order.push_back({steps_of[id], id});
+  }
+  Cut cut;
+  if (!order.empty()) cut = cut_window(order);
+  w.tile_depth = cut.tile_depth;
+  const BatchTileShape shape = batch_tile_shape<T>();
+  for (auto& o : order) {
+    const int depth = cut.tile_depth ? cut.tile_depth : insts_[o.second].depth;
+    o.first = (o.first + depth - 1) / depth;
   }
   std::stable_sort(order.begin(), order.end(),
                    [](const std::pair<int, int>& a, const std::pair<int, int>& b) {
                      return a.first > b.first;
                    });
   int tile_base = 0;
-  const int rows = order.empty() ? 0 : window_rows(order);
   for (size_t k = 0; k < order.size(); ++k) {
     const Inst& in = insts_[order[k].second];
-    const int seg_len = std::min(in.seg_len ? in.seg_len : rows, in.p.ny);
-    const int nsegs = (in.p.ny + seg_len - 1) / seg_len;
+    const int seg_len = std::min(in.seg_len ? in.seg_len : cut.rows, in.p.ny);
+    const int out_x = shape.cols - 4 * cut.tile_depth, out_y = shape.rows - 4 * cut.tile_depth;
+    const int nstrips = cut.tile_depth ? (in.p.nx + out_x - 1) / out_x : in.nstrips;
+    const int nsegs = cut.tile_depth ? (in.p.ny + out_y - 1) / out_y : (in.p.ny + seg_len - 1) / seg_len;
     BatchInst<T> b;
     b.buf[0] = in.buf[0];
     b.buf[1] = in.buf[1];
@@ -457,9 +502,10 @@ typename Engine<T>::Window Engine<T>::plan_window(int window, const std::vector<
     b.yq = YPairs{};
     if constexpr (std::is_same<T, float>::value) b.yq = make_ypairs(in.c.y);
     b.far_rot = in.p.stype == ST_SOA;
-    b.nstrips = in.nstrips;
+    b.nstrips = nstrips;
     b.nsegs = nsegs;
     b.seg_len = seg_len;
+    b.out_x = out_x;
     b.tile_base = tile_base;
     b.parity = cur[order[k].second];
     b.steps = steps_of[order[k].second];
@@ -474,8 +520,8 @@ typename Engine<T>::Window Engine<T>::plan_window(int window, const std::vector<
     w.inst_steps.push_back(steps_of[order[k].second]);
     w.inst_items.push_back(order[k].first);
     for (int s = 0; s < nsegs; ++s)
-      for (int st = 0; st < in.nstrips; ++st) w.tiles.push_back(BatchTile{(int)k, st, s, 0});
-    tile_base += in.nstrips * nsegs;
+      for (int st = 0; st < nstrips; ++st) w.tiles.push_back(BatchTile{(int)k, st, s, 0});
+    tile_base += nstrips * nsegs;
   }
   w.steps = order.empty() ? 0 : order.front().first;
   w.step_items.assign(w.steps + 1, 0);
@@ -518,9 +564,12 @@ int Engine<T>::launch_window(const Window& w, size_t io, size_t to, size_t so, s
   cudaError_t e = cudaMemsetAsync(d_done_ + doff, 0, sizeof(int) * std::max<size_t>(w.tiles.size(), 1), stream_);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_ctl_ + co, 0, sizeof(BatchCtl), stream_);
   if (e == cudaSuccess)
-    e = launch_batch<T>(d_insts_ + io, d_tiles_ + to, d_items_ + so, w.steps, w.step_items.back(),
-                        d_done_ + doff, d_ctl_ + co, wait_ns_, stall_tile_ + 1, resident_blocks_,
-                        stream_);
+    e = w.tile_depth ? launch_batch_tiles<T>(d_insts_ + io, d_tiles_ + to, d_items_ + so, w.steps,
+                                             w.step_items.back(), w.tile_depth, d_done_ + doff, d_ctl_ + co,
+                                             wait_ns_, stall_tile_ + 1, tile_blocks_, stream_)
+                     : launch_batch<T>(d_insts_ + io, d_tiles_ + to, d_items_ + so, w.steps, w.step_items.back(),
+                                       d_done_ + doff, d_ctl_ + co, wait_ns_, stall_tile_ + 1, resident_blocks_,
+                                       stream_);
   stall_tile_ = -1;  // the hook stalls one window
   return e == cudaSuccess ? LE2D_OK : LE2D_ECUDA;
 }

@@ -125,13 +125,18 @@ class Engine {
     std::vector<int> inst_steps;  // time steps of each instance in the window
     std::vector<int> inst_items;  // work-item steps of each instance (ceil(steps / depth))
     int steps = 0;                // work-item steps of the window
+    int tile_depth = 0;           // steps per item on block tiles; 0: strips
   };
   // done_steps / cur: each instance's steps so far and current buffer before the window.
   Window plan_window(int window, const std::vector<long long>& done_steps,
                      const std::vector<int>& cur) const;
-  // Tile height of the instances without one of their own, for a window in which instance
-  // order[k].second runs order[k].first work items.
-  int window_rows(const std::vector<std::pair<int, int>>& order) const;
+  // How a window in which instance steps[k].second runs steps[k].first time steps is cut: block
+  // tiles of tile_depth steps per item, or strips, `rows` the tile height of the instances
+  // without one of their own.
+  struct Cut {
+    int tile_depth = 0, rows = 0;
+  };
+  Cut cut_window(const std::vector<std::pair<int, int>>& steps) const;
   int ensure_scratch(size_t insts, size_t tiles, size_t items, size_t done, size_t ctls);
   int launch_window(const Window& w, size_t inst_off, size_t tile_off, size_t item_off,
                     size_t done_off, size_t ctl_off);
@@ -149,10 +154,11 @@ class Engine {
   unsigned long long wait_ns_ = 2000000000ULL;
   int stall_tile_ = -1;  // test hook from LE2D_TEST_STALL_TILE (see launch_batch): in the
                          // engine's first window only
+  bool stall_strips_ = false;
   int seg_len_ = 0;  // explicit tile height (set_seg_len)
   int depth_set_ = 0;
   bool use_tuned_ = true;
-  int resident_blocks_ = 0;
+  int resident_blocks_ = 0, tile_blocks_ = 0;  // of the strips' and the block tiles' kernel
   long long node_updates_ = 0;
   // device scratch of the persistent launches (work lists, counters)
   BatchInst<T>* d_insts_ = nullptr;

@@ -138,6 +138,7 @@ struct BatchInst {
   YPairs yq;             // FP32: c.y as pairs for the packed y-pipeline
   int far_rot;           // le_step_soa far-end rows
   int nstrips, nsegs, seg_len;
+  int out_x;             // block tiles: columns a tile writes (nstrips across, nsegs down)
   int tile_base;         // index of the instance's first tile in the tile list and done[]
   int parity;            // buffer holding the state at window step 0
   int steps;             // steps of this instance in the window
@@ -185,6 +186,23 @@ cudaError_t launch_batch(const BatchInst<T>* insts, const BatchTile* tiles,
                          const long long* step_items, int nsteps, long long total_items, int* done,
                          BatchCtl* ctl, unsigned long long wait_ns, int stall_plus1,
                          int resident_blocks, cudaStream_t s);
+
+// The same window on block tiles (tile.cuh): each work item advances a tile by up to `depth` steps.
+// A tile's shape, and the most steps per item for which a tile's halo stays within the tiles
+// around it.
+struct BatchTileShape {
+  int cols, rows, max_depth;
+  double a, b;    // an item's time, a + b x steps (us)
+  double loaded;  // and how much more it is when every SM has one
+};
+template <typename T>
+BatchTileShape batch_tile_shape();
+template <typename T>
+int batch_tile_resident_blocks(int device);
+template <typename T>
+cudaError_t launch_batch_tiles(const BatchInst<T>* insts, const BatchTile* tiles, const long long* step_items,
+                               int nsteps, long long total_items, int depth, int* done, BatchCtl* ctl,
+                               unsigned long long wait_ns, int stall_plus1, int resident_blocks, cudaStream_t s);
 
 // FP64 diagnostics: out[0] energy sum (before the h.x*h.y factor), out[1..5] sum of
 // squares, out[6..10] max |value| (as ordered bit patterns).  out must be zeroed first.

@@ -45,8 +45,8 @@ __global__ void __launch_bounds__(W * 32, 1) block_tile_kernel(const __grid_cons
   // rows shared out evenly (le_step_soa's far end needs at least 3 in the last tile)
   const int oy0 = (int)((long long)ty * p.g.ny / p.nty), oy1 = (int)((long long)(ty + 1) * p.g.ny / p.nty);
   // loads past L1: under a programmatic launch the data may be older there
-  march::block_tile<T, V, R, W, true>(p.g, p.c.x, ycons(p), ox0, ox1, oy0, oy1, p.depth, p.steps,
-                                      reinterpret_cast<T*>(smem_raw));
+  march::block_tile<T, V, R, W, true, false>(p.g, p.c.x, ycons(p), ox0, ox1, oy0, oy1, p.depth, p.steps,
+                                             reinterpret_cast<T*>(smem_raw), march::BlockTap<T>{nullptr, -1, 1, 1});
 }
 
 // Tile shapes: V columns per lane, R rows per warp, W warps; A and B of the launch time above

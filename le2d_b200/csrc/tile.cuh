@@ -85,12 +85,23 @@ __device__ __forceinline__ void block_sweep_y(T (&f)[R][NF][V], const T* buf, co
   }
 }
 
+// A receiver line of a batched instance: vx and vy of `row` after every `every` steps, the next
+// sample `until` (1 .. every) steps ahead, at out[0 .. pitch) and out[pitch .. 2 pitch); the
+// samples follow each other.
+template <typename T>
+struct BlockTap {
+  T* out;
+  int row, every, until;
+};
+
 // Advances the tile that writes columns [ox0, ox1), rows [oy0, oy1) by `steps` steps; its
 // first column and row lie 2 * depth before ox0 and oy0 (depth >= steps; ox0 a multiple of V).
-// ox1 - ox0 + 4 depth <= 32 V and oy1 - oy0 + 4 depth <= R W.  Called by the whole block.
-template <typename T, int V, int R, int W, bool COHERENT, typename CY>
+// ox1 - ox0 + 4 depth <= 32 V and oy1 - oy0 + 4 depth <= R W.  TAP: records the tile's part of a
+// receiver line.  Called by the whole block.
+template <typename T, int V, int R, int W, bool COHERENT, bool TAP, typename CY>
 __device__ __forceinline__ void block_tile(const GridRef<T>& g, const Sweep<T>& cx, const CY& cy, int ox0,
-                                           int ox1, int oy0, int oy1, int depth, int steps, T* smem) {
+                                           int ox1, int oy0, int oy1, int depth, int steps, T* smem,
+                                           BlockTap<T> tap) {
   using VT = typename Vec<T, V>::type;
   constexpr int kIn = 32 * V;
   constexpr int kBuf = R * W * kXchg * kIn;
@@ -146,6 +157,18 @@ __device__ __forceinline__ void block_tile(const GridRef<T>& g, const Sweep<T>& 
     if (j0 < yhi && j0 + R > ylo)
       block_sweep_y<T, V, R>(f, buf + lane * V, rows, cy);
     buf = buf == smem ? smem + kBuf : smem;
+    if (TAP && tap.out != nullptr && --tap.until == 0) {
+      tap.until = tap.every;
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        if (j0 + i == tap.row && tap.row >= oy0 && tap.row < oy1 && col0 >= ox0 && col0 < ox1 &&
+            in_line(col0, V, g.pitch)) {
+          *reinterpret_cast<VT*>(tap.out + col0) = pack(f[i][VX]);
+          *reinterpret_cast<VT*>(tap.out + g.pitch + col0) = pack(f[i][VY]);
+        }
+      }
+      tap.out += 2 * g.pitch;
+    }
   }
 
 #pragma unroll
