@@ -231,7 +231,7 @@ long long row_pitch(int nx) { return le2d::row_pitch_elems(nx); }
 // measured on large grids (FP32: two steps per launch on producer / consumer warp pairs,
 // 4 columns per lane, 16 warps per SM, one pair per block, boundary tiles first, interior
 // tiles on the lean loops; FP64: one step per launch, 2 columns per lane, boundary tiles
-// first, interior tiles on the lean one-step loop in 128 registers, 16 warps per SM -- the
+// first, interior tiles on the lean one-step loop in 168 registers, 12 warps per SM -- the
 // FP64 two-step variants measured slower).
 int default_variant() {
   static const int v = [] {  // read once, thread-safely

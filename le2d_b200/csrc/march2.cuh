@@ -91,10 +91,9 @@ __device__ __forceinline__ void ring_output(const YPipe<T, V>& yp, T (&out)[NF][
   row_output(yp, out, ring + (slot == 2 ? 0 : slot + 1) * kRow, cy);
 }
 
-// The three rows of a ring as the pairs' lean loops hold them: rows m, m-1 and m-2, turned by one
+// The three rows of a ring as the lean loops hold them: rows m, m-1 and m-2, turned by one
 // after every row instead of found from a slot number (132.7 -> 130.3 instructions per
-// node-update; 8192^2 323.4 -> 319.9, 4096^2 89.4 -> 87.9 us a step).  The FP64 one-step loop, at
-// its 128 registers, lost 3 % by it.
+// node-update; 8192^2 323.4 -> 319.9, 4096^2 89.4 -> 87.9 us a step).
 template <typename T>
 struct RingRows {
   T *cur, *prev, *prev2;

@@ -206,7 +206,7 @@ template <> struct VariantCfg<double, 11> { static constexpr int V = 2, MINB = 3
 template <> struct VariantCfg<double, 12> { static constexpr int V = 2, MINB = 6, NPF = 2, D = 2, P = 1, W = 2, F = 1; };
 template <> struct VariantCfg<double, 13> { static constexpr int V = 2, MINB = 6, NPF = 2, D = 2, P = 1, W = 2, F = 2; };
 template <> struct VariantCfg<double, 14> { static constexpr int V = 2, MINB = 2, NPF = 2, D = 1, P = 0, W = 4, F = 2; };
-template <> struct VariantCfg<double, 15> { static constexpr int V = 2, MINB = 4, NPF = 2, D = 1, P = 0, W = 4, F = 2; };
+template <> struct VariantCfg<double, 15> { static constexpr int V = 2, MINB = 3, NPF = 2, D = 1, P = 0, W = 4, F = 2; };
 constexpr int kVariants = 16;
 
 template <typename T, int VAR>
