@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(W * 32, 1)
       tap = march::BlockTap<T>{I.trace + samples * 2 * I.pitch, I.trace_row, I.trace_every,
                                (int)((samples + 1) * I.trace_every - before)};
     }
-    march::block_tile<T, V, R, W, true, true>(g, s_c.x, s_c.y, ox0, ox1, oy0, oy1, depth, nadv,
+    march::block_tile<T, V, R, W, true, true, false>(g, s_c.x, s_c.y, ox0, ox1, oy0, oy1, depth, nadv,
                                               reinterpret_cast<T*>(smem_raw), tap);
     __syncthreads();  // the tile's new state is written, its constants read
     const int tile_id = I.tile_base + bt.seg * I.nstrips + bt.strip;

@@ -1,18 +1,20 @@
 // Small grids: several time steps per launch on block tiles (tile.cuh).
 //
 // What bounds it.  A launch costs A + B x steps per wave of tiles: A (launch, tile and halo
-// read from L2, instruction fetch, write) is 2.6 to 6.3 us, and a step's B follows the nodes
+// read from L2, instruction fetch, write) is 2.1 to 5.8 us, and a step's B follows the nodes
 // of a tile.  More steps per launch share A but widen the halo that neighbouring tiles compute
 // twice, so the best tile and depth depend on the grid, and plan_tiles() takes them from a
 // table of measured A and B.  Measured (us a step, this path / the strip march as it was
-// planned before, 32-row segments): FP32 100 x 67 1.4 / 18.2, 256^2 1.8 / 18.4, 512^2 3.5 /
-// 18.5, 700 x 600 4.9 / 18.5, 1200 x 900 11.9 / 20.3; FP64 100 x 67 2.9 / 24.0, 256^2 4.3 /
-// 24.4, 512^2 9.6 / 24.6, 700 x 600 16.3 / 24.6.
+// planned before, 32-row segments): FP32 100 x 67 1.2 / 18.2, 256^2 1.6 / 18.4, 512^2 3.3 /
+// 18.5, 700 x 600 4.5 / 18.5, 1200 x 900 11.6 / 20.3; FP64 100 x 67 2.6 / 24.0, 256^2 4.1 /
+// 24.4, 512^2 9.4 / 24.6, 700 x 600 16.1 / 24.6.
 //
 // Launches are programmatic: a launch's blocks may come up while the one before drains and
-// wait for it (griddepcontrol) before they read.  Without it every launch of a stream took
-// whole multiples of about 2 us (100 x 67 1.4 against 2.1 us a step, 512^2 3.9 against 4.3); a
-// captured graph did about as well but has to be captured first.
+// wait for it (griddepcontrol) only before they read, with their addresses, masks and row table
+// formed: waiting at the kernel's start cost 0.4 to 0.9 us a launch (100 x 67 1.41 / 1.23, 512^2
+// 3.48 / 3.34 us a step).  Without programmatic launches every launch of a stream took whole
+// multiples of about 2 us (100 x 67 1.4 against 2.1 us a step, 512^2 3.9 against 4.3); a captured
+// graph did about as well but has to be captured first.
 #include <atomic>
 #include <cmath>
 #include <type_traits>
@@ -39,14 +41,14 @@ template <typename T, int V, int R, int W>
 __global__ void __launch_bounds__(W * 32, 1) block_tile_kernel(const __grid_constant__ TileParams<T> p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cudaTriggerProgrammaticLaunchCompletion();
-  cudaGridDependencySynchronize();  // the launch before wrote the state read here
   const int tx = blockIdx.x % p.ntx, ty = blockIdx.x / p.ntx;
   const int ox0 = tx * p.out_x, ox1 = min(ox0 + p.out_x, p.g.nx);
   // rows shared out evenly (le_step_soa's far end needs at least 3 in the last tile)
   const int oy0 = (int)((long long)ty * p.g.ny / p.nty), oy1 = (int)((long long)(ty + 1) * p.g.ny / p.nty);
   // loads past L1: under a programmatic launch the data may be older there
-  march::block_tile<T, V, R, W, true, false>(p.g, p.c.x, ycons(p), ox0, ox1, oy0, oy1, p.depth, p.steps,
-                                             reinterpret_cast<T*>(smem_raw), march::BlockTap<T>{nullptr, -1, 1, 1});
+  march::block_tile<T, V, R, W, true, false, true>(p.g, p.c.x, ycons(p), ox0, ox1, oy0, oy1, p.depth, p.steps,
+                                                   reinterpret_cast<T*>(smem_raw),
+                                                   march::BlockTap<T>{nullptr, -1, 1, 1});
 }
 
 // Tile shapes: V columns per lane, R rows per warp, W warps; A and B of the launch time above
@@ -64,11 +66,11 @@ template <typename T>
 struct Shapes;
 template <>
 struct Shapes<float> {
-  static constexpr TileShape s[] = {{2, 4, 16, 4.7, 2.62}, {2, 4, 12, 4.43, 1.68}, {2, 2, 16, 4.06, 0.98}, {2, 2, 8, 2.6, 0.62}};
+  static constexpr TileShape s[] = {{2, 4, 16, 4.0, 2.62}, {2, 4, 12, 3.6, 1.68}, {2, 2, 16, 3.3, 0.98}, {2, 2, 8, 2.1, 0.62}};
 };
 template <>
 struct Shapes<double> {
-  static constexpr TileShape s[] = {{2, 4, 12, 6.34, 6.36}, {2, 2, 12, 3.55, 3.13}, {2, 1, 16, 3.0, 2.05}};
+  static constexpr TileShape s[] = {{2, 4, 12, 5.8, 6.36}, {2, 2, 12, 3.1, 3.13}, {2, 1, 16, 2.5, 2.05}};
 };
 constexpr int kMaxDepth = 6;
 
@@ -125,9 +127,9 @@ cudaError_t launch_shape(int shape, const TileParams<T>& p, int blocks, cudaStre
 // fastest of all shapes and depths measured on each of the grids named above and 900^2.
 // The strip march's time per step is fitted on 700 x 600 to 2048^2 (its best segments, whole or
 // in halves): FP32 7.0 + 5.45 us per million nodes (900^2 12.2, 1200 x 900 12.7, 2048^2 29.9
-// us), FP64 11 + 17.8 us (19.3, 30.4, 85 us).  So FP32 grids cross over at about 1.2 million
-// nodes (1200 x 900 11.9 on tiles, 12.7 on strips; 1500^2 23 and 20.7), FP64 ones at 0.6
-// million (700 x 600 16.3 and 19.3; 900^2 27.5 and 25.0).
+// us), FP64 11 + 17.8 us (700 x 600 19.3, 1200 x 900 30.4, 2048^2 85 us).  So FP32 grids cross over
+// at about 1.2 million nodes (1200 x 900 11.6 on tiles, 12.7 on strips; 1500^2 23 and 20.7), FP64
+// ones at 0.6 million (700 x 600 16.1 and 19.3; 900^2 27.5 and 25.0).
 template <typename T>
 TilePlan plan_tiles(int nx, int ny, int sms) {
   TilePlan best;

@@ -97,8 +97,9 @@ struct BlockTap {
 // Advances the tile that writes columns [ox0, ox1), rows [oy0, oy1) by `steps` steps; its
 // first column and row lie 2 * depth before ox0 and oy0 (depth >= steps; ox0 a multiple of V).
 // ox1 - ox0 + 4 depth <= 32 V and oy1 - oy0 + 4 depth <= R W.  TAP: records the tile's part of a
-// receiver line.  Called by the whole block.
-template <typename T, int V, int R, int W, bool COHERENT, bool TAP, typename CY>
+// receiver line.  WAIT: waits for the launch before, after what does not depend on it.  Called by
+// the whole block.
+template <typename T, int V, int R, int W, bool COHERENT, bool TAP, bool WAIT, typename CY>
 __device__ __forceinline__ void block_tile(const GridRef<T>& g, const Sweep<T>& cx, const CY& cy, int ox0,
                                            int ox1, int oy0, int oy1, int depth, int steps, T* smem,
                                            BlockTap<T> tap) {
@@ -110,6 +111,13 @@ __device__ __forceinline__ void block_tile(const GridRef<T>& g, const Sweep<T>& 
   const int j0 = y_tile + warp * R;
   const int col0 = ox0 - 2 * depth + lane * V;
   const bool col_in = col0 >= 0 && col0 < g.nx;
+
+  float em[V + 1];  // FP32: face e lies between columns col0 + e - 1 and col0 + e
+#pragma unroll
+  for (int e = 0; e <= V; ++e) em[e] = col0 + e >= 1 && col0 + e < g.nx ? 1.0f : 0.0f;
+  BlockRows<R> rows;
+  rows.set(j0, y_tile, R * W, g.ny, g.far_rot);
+  if constexpr (WAIT) cudaGridDependencySynchronize();  // the launch before wrote the state read here
 
   T f[R][NF][V];
 #pragma unroll
@@ -127,12 +135,7 @@ __device__ __forceinline__ void block_tile(const GridRef<T>& g, const Sweep<T>& 
       for (int e = 1; e < V; ++e) f[i][k][e] = col0 + e < g.nx ? f[i][k][e] : (T)0;
     }
   }
-  float em[V + 1];  // FP32: face e lies between columns col0 + e - 1 and col0 + e
-#pragma unroll
-  for (int e = 0; e <= V; ++e) em[e] = col0 + e >= 1 && col0 + e < g.nx ? 1.0f : 0.0f;
 
-  BlockRows<R> rows;
-  rows.set(j0, y_tile, R * W, g.ny, g.far_rot);
   T* buf = smem;
   for (int s = 0; s < steps; ++s) {
     // rows the remaining steps need of this one, and of its x-sweep
