@@ -505,8 +505,7 @@ unsigned long long check_violations_batch() {
                                              const long long*, int, long long, int, int*,       \
                                              BatchCtl*, unsigned long long, int, int,           \
                                              cudaStream_t);
-LE2D_INST(float)
-LE2D_INST(double)
+LE2D_INST(real)
 #undef LE2D_INST
 
 }  // namespace le2d

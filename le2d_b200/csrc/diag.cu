@@ -107,9 +107,7 @@ cudaError_t launch_diag(const T* soa, int nx, int ny, long long pitch, long long
   return cudaGetLastError();
 }
 
-template cudaError_t launch_diag<float>(const float*, int, int, long long, long long, double,
-                                        double, double, double, double*, cudaStream_t);
-template cudaError_t launch_diag<double>(const double*, int, int, long long, long long, double,
-                                         double, double, double, double*, cudaStream_t);
+template cudaError_t launch_diag<real>(const real*, int, int, long long, long long, double,
+                                       double, double, double, double*, cudaStream_t);
 
 }  // namespace le2d

@@ -180,8 +180,7 @@ cudaError_t launch_vtk_speed(const T* soa, int nx, int ny, long long pitch, long
                                           cudaStream_t);                                           \
   template cudaError_t launch_vtk_speed<T>(const T*, int, int, long long, long long, unsigned*,  \
                                            cudaStream_t);
-LE2D_INST(float)
-LE2D_INST(double)
+LE2D_INST(real)
 #undef LE2D_INST
 
 }  // namespace le2d

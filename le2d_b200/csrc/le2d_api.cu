@@ -80,7 +80,7 @@ struct DevTask {
   cudaEvent_t hev[3][2] = {{nullptr, nullptr}, {nullptr, nullptr}, {nullptr, nullptr}};
   cudaEvent_t fork_ev = nullptr;
   long long hk = 0;
-  bool seq_open = false;  // le_step calls left a sequence of launches in halves open (close_sequence)
+  bool seq_open = false;  // le_step calls left a sequence of launches in halves open (flush_pending joins it)
 };
 
 constexpr int kGraphSteps = 64;  // even, so a replay leaves the current buffer unchanged

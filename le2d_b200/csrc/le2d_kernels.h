@@ -1,11 +1,14 @@
 // Launchers of the device kernels (host side).  All take device pointers to the
-// SoA state: field k, row j, column i at base[k * plane + j * pitch + i].
+// SoA state: field k, row j, column i at base[k * plane + j * pitch + i].  Each library holds
+// the instances of its own precision (`real`) only: with both, the first task of a process
+// loaded twice the code.
 #pragma once
 
 #include <cuda_runtime.h>
 #include <stddef.h>
 
 #include "le2d_device.cuh"
+#include "le_core.h"
 
 namespace le2d {
 

@@ -527,8 +527,7 @@ unsigned long long check_violations_fused() {
                                             const StepConsts<T>&, int, const FusedPlan&,        \
                                             const PairCtl&, int, int, const int*, const int*,   \
                                             cudaStream_t);
-LE2D_INST(float)
-LE2D_INST(double)
+LE2D_INST(real)
 #undef LE2D_INST
 
 }  // namespace le2d

@@ -136,11 +136,8 @@ cudaError_t launch_split_sweep(int axis, const T* src, T* dst, int nx, int ny, l
   return cudaGetLastError();
 }
 
-template cudaError_t launch_split_sweep<float>(int, const float*, float*, int, int, long long,
-                                               long long, const Sweep<float>&, float, float, int,
-                                               cudaStream_t);
-template cudaError_t launch_split_sweep<double>(int, const double*, double*, int, int, long long,
-                                                long long, const Sweep<double>&, double, double,
-                                                int, cudaStream_t);
+template cudaError_t launch_split_sweep<real>(int, const real*, real*, int, int, long long,
+                                              long long, const Sweep<real>&, real, real, int,
+                                              cudaStream_t);
 
 }  // namespace le2d

@@ -191,8 +191,7 @@ unsigned long long check_violations_tiles() {
   template TilePlan plan_tiles<T>(int, int, int);                                                 \
   template cudaError_t launch_tiles<T>(const T*, T*, int, int, long long, long long,              \
                                        const StepConsts<T>&, int, const TilePlan&, int, cudaStream_t);
-LE2D_INST(float)
-LE2D_INST(double)
+LE2D_INST(real)
 #undef LE2D_INST
 
 }  // namespace le2d
