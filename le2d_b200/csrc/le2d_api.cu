@@ -15,6 +15,8 @@
 // never aborts or exits: it prints the cause on stderr and keeps the first error
 // per task (le2d_last_error).  There is no CPU fallback: without a device, steps
 // fail with LE2D_ENODEV.
+#include <cuda.h>
+
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -26,6 +28,7 @@
 #include "consts.h"
 #include "le2d.h"
 #include "le2d_kernels.h"
+#include "rows_copy.h"
 
 namespace {
 
@@ -37,6 +40,7 @@ using le2d::Sweep;
 constexpr int kMinSeg = 16;  // shortest row segment of the fused kernel
 
 struct DevTask {
+  int device = 0;  // the device that was current when the task was made
   int nx = 0, ny = 0;
   long long pitch = 0, plane = 0;
   T* mem = nullptr;
@@ -800,6 +804,7 @@ void le_init_task(le_task* task, const real dt, const le_vec2 h, const le_materi
   if (n.x < 3 || n.y < 3) record(d, LE2D_EINVAL, "le_init_task: the scheme needs n.x, n.y >= 3");
   if (stype != ST_AOS && stype != ST_SOA) record(d, LE2D_EINVAL, "le_init_task: unknown stype");
   if (d->has_device) {
+    cudaGetDevice(&d->device);
     d->pitch = row_pitch(n.x);
     d->plane = d->pitch * n.y;
     const size_t dbytes = sizeof(T) * 2 * 5 * (size_t)d->plane;
@@ -1150,18 +1155,34 @@ int le2d_diagnostics(le_task* task, le2d_diag_t* out) {
 
 namespace {
 
-// Whether a buffer a caller hands to le2d_rows_out / le2d_rows_in is memory of the current
-// device, aligned to T, which one kernel copies; anything else a copy call takes (another
-// device's memory, page-locked host memory) goes through one.
-bool copied_by_kernel(const T* buf) {
+// Whether one kernel copies `bytes` between the task's state and a buffer a caller hands to
+// le2d_rows_out / le2d_rows_in (rows_by_kernel).
+bool copied_by_kernel(const DevTask* d, const T* buf, size_t bytes) {
+  using Range = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+  static const Range range_of = [] {  // the driver's, looked up once, thread-safely
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return (Range)f;
+  }();
   cudaPointerAttributes a;
+  CUdeviceptr base = 0;
+  le2d::RowsBuffer b;
   int dev = -1;
-  if ((uintptr_t)buf % sizeof(T) != 0 || cudaGetDevice(&dev) != cudaSuccess ||
-      cudaPointerGetAttributes(&a, buf) != cudaSuccess) {
+  if (!range_of || cudaGetDevice(&dev) != cudaSuccess || cudaPointerGetAttributes(&a, buf) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  return a.type == cudaMemoryTypeDevice && a.device == dev;
+  b.device_memory = a.type == cudaMemoryTypeDevice;
+  if (!b.device_memory || range_of(&base, &b.extent, (CUdeviceptr)(uintptr_t)buf) != CUDA_SUCCESS) return false;
+  b.device = a.device;
+  b.at = (uintptr_t)buf;
+  b.base = (uintptr_t)base;
+  return le2d::rows_by_kernel(b, bytes, sizeof(T), d->device, dev);
 }
 
 // Rows [row0, row0 + nrows) of the task's state <-> a caller's device buffer laid out
@@ -1179,7 +1200,7 @@ int copy_rows(le_task* task, int row0, int nrows, T* dev_buf, void* stream, bool
   cudaError_t e = cudaEventRecord(d->ev[0], d->stream);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(s, d->ev[0], 0);
   T* first = d->buf[d->cur] + (long long)row0 * d->pitch;
-  const bool kernel = e == cudaSuccess && copied_by_kernel(dev_buf);
+  const bool kernel = e == cudaSuccess && copied_by_kernel(d, dev_buf, sizeof(T) * 5 * (size_t)nrows * d->nx);
   if (kernel) e = le2d::launch_copy_rows<T>(first, dev_buf, d->nx, nrows, d->pitch, d->plane, out, s);
   for (int k = 0; k < 5 && e == cudaSuccess && !kernel; ++k) {
     T* state = first + k * d->plane;
