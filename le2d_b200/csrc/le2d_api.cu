@@ -649,6 +649,7 @@ int run_steps(le_task* task, int nsteps, bool soa_entry, float* ms) {
         rc = capture_steps(d, c, far_rot, halves, &graph);
         if (rc) return rc;
       }
+      if (d->method == LE2D_METHOD_FUSED && d->plan.warps_per_task == 2) d->pairs_queued = true;
       e = cudaGraphLaunch(graph, d->stream);
       if (e != cudaSuccess) return record(d, LE2D_ECUDA, "graph launch", e);
       left -= kGraphSteps;
