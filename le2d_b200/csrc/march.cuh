@@ -254,9 +254,11 @@ __device__ __forceinline__ float2 ratio2(float2 a, float2 b) { return mul2(a, rc
 // Face e (0..V) lies between node e-1 and node e of the lane; the neighbour lanes supply the
 // fields of nodes -1 and V and the flux terms of their edge nodes.
 //
-// MASK: `em[e]` (0 or 1) multiplies the differences of face e, for lanes that hold columns at
-// or beyond the grid's ends (block tiles, tile.cuh): a face with a clamped column has two equal
-// sides, so its differences are 0, and every term the neighbours take from it is then 0 too.
+// MASK: `em[e]` (0 or 1) multiplies the field differences of face e, for lanes that hold columns
+// at or beyond the grid's ends (block tiles, tile.cuh): a face with a clamped column has two equal
+// sides, so its differences are 0, and every term the neighbours take from it is then 0 too.  The
+// field differences, not those of the invariants: a stress divided by rho c may leave the type's
+// range where the stress does not, and 0 times that is no 0.
 template <int V, bool MASK = false>
 __device__ __forceinline__ void sweep_x_lane_packed(float (&f)[NF][V], const Sweep<float>& c,
                                                     const float (&em)[V + 1] = {}) {
@@ -279,14 +281,14 @@ __device__ __forceinline__ void sweep_x_lane_packed(float (&f)[NF][V], const Swe
     const float nsx = e < V ? f[SXX][e] : rf[1], psx = e > 0 ? f[SXX][e - 1] : lf[1];
     const float nvy = e < V ? f[VY][e] : rf[2], pvy = e > 0 ? f[VY][e - 1] : lf[2];
     const float nxy = e < V ? f[SXY][e] : rf[3], pxy = e > 0 ? f[SXY][e - 1] : lf[3];
-    const float2 dv = f2(nvx - pvx, nvy - pvy);
-    const float2 ds = f2(nsx - psx, nxy - pxy);
+    float2 dv = f2(nvx - pvx, nvy - pvy);
+    float2 ds = f2(nsx - psx, nxy - pxy);
+    if constexpr (MASK) {
+      dv = mul2(dv, f2(em[e], em[e]));
+      ds = mul2(ds, f2(em[e], em[e]));
+    }
     dr[e] = fma2(neg2(ds), c.irp, dv);
     dl[e] = fma2(ds, c.irp, dv);
-    if constexpr (MASK) {
-      dr[e] = mul2(dr[e], f2(em[e], em[e]));
-      dl[e] = mul2(dl[e], f2(em[e], em[e]));
-    }
   }
   float2 na[V], b[V];  // (-A1, -A3) and (B2, B4) of node v
   {  // right-moving (w1, w3): psi_v = psi(P_v / P_{v+1}), -t_v = D_{v+1} - psi_v D_{v+1}
