@@ -77,17 +77,18 @@ int le2d_set_variant(le_task *task, int variant, int seg_len);
 /* out[8] = {variant, columns per lane, segment rows, strips, tiles, blocks,
  * temporal-block depth, warps per tile (2: producer / consumer warp pair)}. */
 int le2d_get_plan(const le_task *task, int *out);
-/* Small grids on their default plan (no variant or segment length asked for) run several time
- * steps per launch on block tiles instead of the strip plan above, which stays the one
- * le2d_get_plan reports; results are bitwise the same.  out[5] = {steps per launch (0: the task
- * runs its strip plan), columns and rows of a tile with its halo, tiles across, tiles down}.
+/* Small grids on their default plan (no variant or segment length asked for, neither
+ * LE2D_FUSED_VARIANT nor LE2D_HALVES set) run several time steps per launch on block tiles
+ * instead of the strip plan above, which stays the one le2d_get_plan reports; results are
+ * bitwise the same.  out[5] = {steps per launch (0: the task runs its strip plan), columns and
+ * rows of a tile with its halo, tiles across, tiles down}.
  * le_step / le_step_soa calls share launches then, as under a two-step plan. */
 int le2d_block_tiles(const le_task *task, int *out);
 /* *parts = kernel launches per fused launch of the grid: 1, or 3 when the task's launches go
  * in halves (the band of rows around the middle row on a high-priority stream and the rows
  * above and below it on two more streams, waiting for each other only where their stencils
  * meet -- chosen per grid and plan where it measured faster; LE2D_HALVES=1 / 0 forces it on
- * / off for tasks created afterwards). */
+ * / off, on the strip plan, for every task of a process started with it). */
 int le2d_launch_parts(const le_task *task, int *parts);
 
 /* Autotuner: times every compiled fused-kernel variant (columns per lane, register bound,

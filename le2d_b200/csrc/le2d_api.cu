@@ -248,8 +248,8 @@ int default_variant() {
 }
 
 // Whether small grids run on block tiles by default: not when the environment asks for a
-// variant of the strip march or for its launches in halves.
-bool default_tiles() { return getenv("LE2D_FUSED_VARIANT") == nullptr && halves_mode() != 1; }
+// variant of the strip march, or for its launches in halves or whole.
+bool default_tiles() { return getenv("LE2D_FUSED_VARIANT") == nullptr && halves_mode() < 0; }
 
 void drop_graphs(DevTask* d) {
   for (cudaGraphExec_t& g : d->graph) {
