@@ -768,15 +768,23 @@ bool Engine<T>::failed(int id) const {
 }
 
 template <typename T>
-int Engine<T>::harvest_fields(int id, T* out) {
-  if (id < 0 || id >= (int)insts_.size() || !out) return LE2D_EINVAL;
+int Engine<T>::harvest_fields(int id, const Parts& out) {
+  if (id < 0 || id >= (int)insts_.size() || out.empty()) return LE2D_EINVAL;
   const Inst& in = insts_[id];
   if (!in.live || in.failed || !finished(id)) return in.failed ? LE2D_ETIMEOUT : LE2D_ESTATE;
-  if (!in.unpacked) return fields(id, out);  // no window ran (zero steps)
-  cudaError_t e = cudaMemcpyAsync(out, in.buf[in.cur ^ 1], sizeof(T) * 5 * (size_t)in.p.nx * in.p.ny,
-                                  cudaMemcpyDeviceToHost, copy_);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(copy_);
-  return e == cudaSuccess ? LE2D_OK : LE2D_ECUDA;
+  const char* src = reinterpret_cast<const char*>(in.buf[in.cur ^ 1]);
+  cudaError_t e = cudaSuccess;
+  if (!in.unpacked) {  // no window ran (zero steps)
+    e = launch_unpack<T>(in.buf[in.cur], in.buf[in.cur ^ 1], in.p.nx, in.p.ny, in.pitch, in.plane,
+                         in.p.stype == ST_AOS, stream_);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
+  }
+  for (size_t k = 0; k < out.size() && e == cudaSuccess; ++k) {
+    e = cudaMemcpyAsync(out[k].first, src, out[k].second, cudaMemcpyDeviceToHost, copy_);
+    src += out[k].second;
+  }
+  const cudaError_t e2 = cudaStreamSynchronize(copy_);
+  return e == cudaSuccess && e2 == cudaSuccess ? LE2D_OK : LE2D_ECUDA;
 }
 
 template <typename T>

@@ -8,6 +8,7 @@
 
 #include <cstddef>
 #include <map>
+#include <utility>
 #include <vector>
 
 #include "le2d.h"
@@ -92,8 +93,10 @@ class Engine {
   int fields(int id, T* out);
   int receivers(int id, T* out, int* nsamples);
   // Results of an instance finished by an earlier window, read on the copy stream, so
-  // they overlap a window in flight (fields: unpacked after the finishing window).
-  int harvest_fields(int id, T* out);
+  // they overlap a window in flight (fields: unpacked after the finishing window), into
+  // memory in parts of (address, bytes).
+  using Parts = std::vector<std::pair<char*, size_t>>;
+  int harvest_fields(int id, const Parts& out);
   int harvest_receivers(int id, T* out, int* nsamples);
   int diagnostics(int id, le2d_diag_t* out);
   // Releases the instance's device memory (its results must have been read).

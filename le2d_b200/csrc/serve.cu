@@ -13,7 +13,9 @@
 //      right after it;
 //   4. while that window runs, read back the results (final fields or receiver traces)
 //      of the solves the previous window finished, on the copy stream, free their
-//      device memory and wake the waiters.
+//      device memory and wake the waiters;
+//   5. with nothing to do, page-lock memory for results like those of the last busy
+//      periods (result_pool.h), a slab at a time, until a request comes.
 // So requests that arrive while others are on the GPU join at the next window, their
 // work overlaps with the others', and uploads and read-backs overlap the windows.  A
 // solve whose tiles' dependency wait gave up fails alone (LE2D_ETIMEOUT); a launch that
@@ -22,17 +24,16 @@
 #include <condition_variable>
 #include <cstdio>
 #include <cstring>
-#include <cstdlib>
 #include <deque>
-#include <iterator>
-#include <map>
 #include <memory>
 #include <mutex>
 #include <thread>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "engine.h"
+#include "result_pool.h"
 
 namespace {
 
@@ -43,93 +44,18 @@ double now_s() {
   return duration<double>(steady_clock::now().time_since_epoch()).count();
 }
 
-// Host memory of the results: page-locked blocks kept for later results once a ticket is
-// released, up to kHeld bytes per server (given back with it).  Page-locking costs more than one
-// result gains by it (0.3 ms per MB), so the pool grows only by what malloc'd results were
-// released before: a server's first results, and what does not fit, are malloc'd and freed with
-// their tickets.  Results read back into fresh pageable memory keep the worker from launching
-// the next window meanwhile (24 requests of 64 to 1024 nodes a side, 25 MB of fields: 25.9 ms a
-// burst, now 11.6 from the third on).
-class ResultPool {
- public:
-  struct Block {
+// Page-locked memory for the results' pool (result_pool.h).
+struct PageLocked {
+  static void* lock(size_t bytes) {
     void* p = nullptr;
-    size_t cap = 0;
-    bool pinned = false;
-  };
-  ~ResultPool() {
-    for (auto& f : free_) cudaFreeHost(f.second);
+    if (cudaHostAlloc(&p, bytes, cudaHostAllocDefault) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
   }
-  Block take(size_t bytes) {
-    bytes = (bytes + kStep - 1) / kStep * kStep;
-    std::lock_guard<std::mutex> lk(mu_);
-    auto it = free_.lower_bound(bytes);
-    if (it != free_.end() && it->first <= 2 * bytes) {
-      Block b{it->second, it->first, true};
-      free_.erase(it);
-      return b;
-    }
-    Block b{nullptr, bytes, false};
-    const bool lock = bytes <= seen_;
-    while (lock && held_ + bytes > seen_ && !free_.empty()) {  // make room: blocks of other sizes
-      auto last = std::prev(free_.end());
-      cudaFreeHost(last->second);
-      held_ -= last->first;
-      free_.erase(last);
-    }
-    if (lock && held_ + bytes <= seen_) {
-      if (cudaHostAlloc(&b.p, bytes, cudaHostAllocDefault) == cudaSuccess) {
-        b.pinned = true;
-        held_ += bytes;
-        return b;
-      }
-      cudaGetLastError();
-    }
-    b.p = malloc(bytes);
-    return b;
-  }
-  void give_back(const Block& b) {
-    std::lock_guard<std::mutex> lk(mu_);
-    if (b.pinned) {
-      free_.emplace(b.cap, b.p);
-    } else {
-      free(b.p);
-      seen_ = seen_ + b.cap < kHeld ? seen_ + b.cap : kHeld;
-    }
-  }
-
- private:
-  static constexpr size_t kStep = (size_t)64 << 10, kHeld = (size_t)256 << 20;
-  std::mutex mu_;
-  std::multimap<size_t, void*> free_;
-  size_t held_ = 0;  // bytes of page-locked blocks, in use and free
-  size_t seen_ = 0;  // bytes of malloc'd results released so far, at most kHeld
+  static void unlock(void* p) { cudaFreeHost(p); }
 };
-
-// A result's block of the pool, which outlives the server's other members with it.
-class Result {
- public:
-  Result() = default;
-  Result(const Result&) = delete;
-  Result& operator=(const Result&) = delete;
-  ~Result() {
-    if (b_.p) pool_->give_back(b_);
-  }
-  // Memory for n values; null when there is none.
-  T* make(const std::shared_ptr<ResultPool>& pool, size_t n) {
-    pool_ = pool;
-    b_ = pool->take(sizeof(T) * (n > 0 ? n : 1));
-    n_ = b_.p ? n : 0;
-    return data();
-  }
-  T* data() const { return (T*)b_.p; }
-  size_t size() const { return n_; }
-
- private:
-  std::shared_ptr<ResultPool> pool_;
-  ResultPool::Block b_;
-  size_t n_ = 0;
-};
+using Pool = le2d::ResultPool<PageLocked>;
+using Result = le2d::PooledResult<PageLocked>;
 
 struct Ticket {
   long long id = 0;
@@ -148,7 +74,7 @@ struct Ticket {
 
 struct le2d_server {
   std::unique_ptr<le2d::Engine<T>> eng;
-  std::shared_ptr<ResultPool> pool = std::make_shared<ResultPool>();
+  std::shared_ptr<Pool> pool = std::make_shared<Pool>();
   int window = 100;
   int max_active = 1024;
   std::mutex mu;
@@ -211,6 +137,12 @@ struct le2d_server {
       if (!added.empty()) cv_done.notify_all();
       if (stop) break;
       if (active.empty() && !eng->in_flight()) {
+        pool->idle();
+        while (!stop && queue.empty() && pool->wants_more()) {  // a slab at a time: requests come first
+          lk.unlock();
+          pool->grow();
+          lk.lock();
+        }
         cv_work.wait(lk, [&] { return stop || !queue.empty(); });
         continue;
       }
@@ -247,11 +179,12 @@ struct le2d_server {
             int n = 0;
             r2 = eng->harvest_receivers(id, nullptr, &n);
             t->nsamples = n;
-            if (r2 == LE2D_OK && !t->result.make(pool, (size_t)n * 2 * t->p.nx)) r2 = LE2D_ENOMEM;
-            if (r2 == LE2D_OK && n > 0) r2 = eng->harvest_receivers(id, t->result.data(), &n);
+            if (r2 == LE2D_OK && !t->result.make(pool, sizeof(T) * (size_t)n * 2 * t->p.nx, true)) r2 = LE2D_ENOMEM;
+            if (r2 == LE2D_OK && n > 0) r2 = eng->harvest_receivers(id, (T*)t->result.parts()[0].first, &n);
           } else {
-            r2 = t->result.make(pool, (size_t)5 * t->p.nx * t->p.ny) ? eng->harvest_fields(id, t->result.data())
-                                                                     : LE2D_ENOMEM;
+            r2 = t->result.make(pool, sizeof(T) * (size_t)5 * t->p.nx * t->p.ny, false)
+                     ? eng->harvest_fields(id, t->result.parts())
+                     : LE2D_ENOMEM;
           }
           status = r2 == LE2D_OK ? 1 : -r2;
         }
@@ -384,8 +317,8 @@ int le2d_server_result(le2d_server* s, long long ticket, real* out, size_t out_e
   // a finished ticket's result no longer changes: copied without holding up the worker
   if (nsamples) *nsamples = t->nsamples;
   if (!out) return LE2D_OK;
-  if (out_elems < t->result.size()) return LE2D_EINVAL;
-  memcpy(out, t->result.data(), sizeof(T) * t->result.size());
+  if (out_elems < t->result.bytes() / sizeof(T)) return LE2D_EINVAL;
+  t->result.copy_to(out);
   return LE2D_OK;
 }
 
@@ -403,10 +336,12 @@ int le2d_server_times(le2d_server* s, long long ticket, double* t_submit, double
 
 int le2d_server_release(le2d_server* s, long long ticket) {
   if (!s) return LE2D_EINVAL;
+  std::shared_ptr<Ticket> t;  // and its result, freed without the server's lock
   std::lock_guard<std::mutex> lk(s->mu);
   auto it = s->tickets.find(ticket);
   if (it == s->tickets.end()) return LE2D_EINVAL;
   if (it->second->status == 0) return LE2D_ESTATE;
+  t = std::move(it->second);
   s->tickets.erase(it);
   return LE2D_OK;
 }

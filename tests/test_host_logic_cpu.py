@@ -38,3 +38,89 @@ def test_rows_copied_by_kernel_only_on_one_device():
         for c in cases)
     out = _run('#include <cstdio>\n#include "rows_copy.h"\nint main() {\n' + body + "}\n")
     assert [int(x) for x in out] == [c[-1] for c in cases]
+
+
+POOL = r"""
+#include <atomic>
+#include <cstdint>
+#include <cstdio>
+#include <thread>
+#include "result_pool.h"
+static std::atomic<int> locks{0}, unlocks{0};
+static bool none = false;
+struct Fake {
+  static void* lock(size_t n) { if (none) return nullptr; ++locks; return malloc(n); }
+  static void unlock(void* p) { ++unlocks; free(p); }
+};
+using Pool = le2d::ResultPool<Fake>;
+using Result = le2d::PooledResult<Fake>;
+constexpr size_t P = Pool::kPiece;
+static std::unique_ptr<Result> get(const std::shared_ptr<Pool>& p, size_t bytes, bool contiguous = false) {
+  auto r = std::make_unique<Result>();
+  if (!r->make(p, bytes, contiguous) || r->bytes() != bytes) { std::printf("no-memory "); return nullptr; }
+  unsigned char v = 0;
+  for (auto& q : r->parts()) for (size_t i = 0; i < q.second; i += 4096) q.first[i] = (char)++v;
+  std::vector<char> out(bytes + 1, 77);
+  r->copy_to(out.data());
+  if (out[bytes] != 77) std::printf("past-the-end ");
+  size_t at = 0; v = 0;
+  for (auto& q : r->parts()) { for (size_t i = 0; i < q.second; i += 4096) if (out[at + i] != (char)++v) std::printf("wrong "); at += q.second; }
+  if (at != bytes) std::printf("size ");
+  return r;
+}
+static void burst(const std::shared_ptr<Pool>& p, std::vector<size_t> sizes) {
+  std::vector<std::unique_ptr<Result>> held;
+  for (size_t n : sizes) held.push_back(get(p, n));
+  p->idle();
+}
+static int grow_all(const std::shared_ptr<Pool>& p) { int n = 0; while (p->wants_more()) { p->grow(); ++n; } return n; }
+int main() {
+  {
+    auto p = std::make_shared<Pool>();
+    const std::vector<size_t> mixed{0, 1, P - 1, P, P + 1, 5 * P + 3, 17 * P};  // 1+1+1+1+2+6+17 = 29 pieces
+    p->idle();
+    burst(p, mixed);
+    std::printf("%d ", grow_all(p));               // one busy period alone: nothing
+    burst(p, mixed);
+    const int before = locks;                      // nothing locked while results come and go
+    std::printf("%d %d ", before, grow_all(p));    // then ceil(29 / 8) slabs
+    burst(p, mixed); burst(p, {40 * P, 3 * P, 9 * P});  // other sizes: no unlocking, no locking
+    std::printf("%d %d ", (int)locks, (int)unlocks);
+    { auto a = get(p, 29 * P); auto b = get(p, 4 * P); auto c = get(p, 2 * P, true); }  // malloc where the pool is short
+    burst(p, {Pool::kHeld + 1}); burst(p, {Pool::kHeld + 1});  // never fits: not asked for
+    std::printf("%d ", grow_all(p));               // 33 at once just now, 52 before: a fifth slab
+    std::vector<size_t> many(3000, P);             // more than the pool may hold
+    burst(p, many); burst(p, many);
+    std::printf("%d %d ", grow_all(p), (int)(locks * Pool::kSlabPieces * P <= Pool::kHeld));
+    none = true; many.assign(8, P);
+    auto held = get(p, P); p.reset();              // a result outlives the server's handle on the pool
+    held.reset();
+    std::printf("%d ", (int)(locks == unlocks));
+  }
+  {
+    auto p = std::make_shared<Pool>();             // page-locking fails: malloc, and no endless tries
+    burst(p, {P}); burst(p, {P});
+    std::printf("%d ", grow_all(p));
+    auto r = get(p, 3 * P);
+  }
+  none = false;
+  {
+    auto p = std::make_shared<Pool>();
+    burst(p, std::vector<size_t>(64, P)); burst(p, std::vector<size_t>(64, P));
+    std::vector<std::thread> th;
+    for (int k = 0; k < 6; ++k) th.emplace_back([&, k] { for (int i = 0; i < 300; ++i) auto r = get(p, (i * 7 + k) % 9 * P / 2); });
+    std::thread worker([&] { for (int i = 0; i < 200; ++i) { p->idle(); if (p->wants_more()) p->grow(); } });
+    for (auto& t : th) t.join();
+    worker.join();
+    grow_all(p);
+    std::printf("%d", (int)(p->take(64).size() == 64));  // every piece came back
+  }
+}
+"""
+
+
+def test_result_pool():
+    """A server's page-locked results (result_pool.h): nothing is locked or unlocked between results,
+    mixed sizes share the pieces, growth waits for two busy periods and ends at the bound."""
+    out = _run(POOL)
+    assert out == ["0", "0", "4", "4", "0", "1", "59", "1", "1", "1", "1"], out
