@@ -165,6 +165,13 @@ int le2d_batch_add(le2d_batch *b, const le2d_problem *p, const real *init, int n
  * le2d_batch_fields / _receivers / _diagnostics return LE2D_ETIMEOUT), the others'
  * results are valid. */
 int le2d_batch_run(le2d_batch *b, int window_steps, float *device_ms);
+/* A window runs on strips or on block tiles, whichever is modelled faster for the instances in it;
+ * results are bitwise the same.  le2d_batch_set_strips: windows with instances added afterwards
+ * run on strips, theirs of `rows` rows (>= 8).  le2d_batch_next_cut: out[2] = {steps per work item
+ * on block tiles (0: strips), rows of a strip's tile of instances without a height of their own}
+ * of the window that would run now (LE2D_ESTATE: no instance has steps left). */
+int le2d_batch_set_strips(le2d_batch *b, int rows);
+int le2d_batch_next_cut(const le2d_batch *b, int window_steps, int *out);
 int le2d_batch_count(const le2d_batch *b);
 /* Final fields of instance `id` (5*nx*ny reals, the problem's layout). */
 int le2d_batch_fields(le2d_batch *b, int id, real *out);

@@ -49,7 +49,7 @@ EXPORTS = [
     "le2d_batch_autotune", "le2d_batch_autotune_reset",
     "le2d_slabs_create", "le2d_slabs_destroy", "le2d_slabs_rows", "le2d_slabs_upload",
     "le2d_slabs_download", "le2d_slabs_step_n", "le2d_slabs_wait", "le2d_selftest_ratio", "le2d_selftest_limiter", "le2d_launch_parts",
-    "le2d_block_tiles",
+    "le2d_block_tiles", "le2d_batch_set_strips", "le2d_batch_next_cut",
     "le2d_rows_out", "le2d_rows_in", "le2d_check_violations",
 ]
 
@@ -160,6 +160,8 @@ class Lib:
         L.le2d_batch_add.argtypes = [ctypes.c_void_p, P(self.le2d_problem), ctypes.c_void_p, ctypes.c_int,
                                      ctypes.c_void_p]
         L.le2d_batch_run.argtypes = [ctypes.c_void_p, ctypes.c_int, P(ctypes.c_float)]
+        L.le2d_batch_set_strips.argtypes = [ctypes.c_void_p, ctypes.c_int]
+        L.le2d_batch_next_cut.argtypes = [ctypes.c_void_p, ctypes.c_int, P(ctypes.c_int)]
         L.le2d_batch_count.argtypes = [ctypes.c_void_p]
         L.le2d_batch_fields.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
         L.le2d_batch_receivers.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, P(ctypes.c_int)]
@@ -469,6 +471,17 @@ class Batch:
         d = self.lib.le2d_diag_t()
         rc = self.lib.lib.le2d_batch_diagnostics(self.h, rid, ctypes.byref(d))
         return rc, {"energy": d.energy, "sumsq": list(d.sumsq), "maxabs": list(d.maxabs)}
+
+    def set_strips(self, rows: int) -> int:
+        return self.lib.lib.le2d_batch_set_strips(self.h, rows)
+
+    def next_cut(self, window_steps: int = 256) -> dict:
+        """How the next window is cut: steps per item on block tiles (0: strips), rows of a strip's tile."""
+        out = (ctypes.c_int * 2)()
+        rc = self.lib.lib.le2d_batch_next_cut(self.h, window_steps, out)
+        if rc:
+            raise RuntimeError(self.lib.strerror(rc))
+        return dict(zip(("tile_depth", "rows"), list(out)))
 
     def set_wait_limit(self, ns: int) -> int:
         return self.lib.lib.le2d_batch_set_wait_limit(self.h, ns)

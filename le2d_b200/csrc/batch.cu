@@ -29,7 +29,7 @@
 // step; the consumer runs the second step on the rows it is handed, writes them, records
 // receiver samples and publishes the tile.  The last item of an odd step count advances
 // one step: the consumer writes the producer's rows as they are.  (le_step_soa's far end reads
-// step A's rows down to ny-7, within the tile above the last one: tiles are at least 8 rows.)
+// step A's rows down to ny-7, within the tile above the last one: tiles are at least 8 rows, Engine::kMinRows.)
 // A producer may claim its next item while its consumer still finishes the last one: all
 // rows of that item are already in the queue, so the consumer finishes without it.
 #include <type_traits>

@@ -142,7 +142,7 @@ size_t Engine<T>::footprint(const le2d_problem& p) {
 
 template <typename T>
 int Engine<T>::set_seg_len(int rows) {
-  if (rows < 1) return LE2D_EINVAL;
+  if (rows < kMinRows) return LE2D_EINVAL;
   seg_len_ = rows;
   return LE2D_OK;
 }
@@ -459,19 +459,37 @@ typename Engine<T>::Cut Engine<T>::cut_window(const std::vector<std::pair<int, i
 }
 
 template <typename T>
-typename Engine<T>::Window Engine<T>::plan_window(int window, const std::vector<long long>& done,
-                                                  const std::vector<int>& cur) const {
-  Window w;
-  std::vector<std::pair<int, int>> order;  // (work-item steps in window, id)
-  std::vector<int> steps_of(insts_.size(), 0);
+std::vector<std::pair<int, int>> Engine<T>::window_steps(int window, const std::vector<long long>& done) const {
+  std::vector<std::pair<int, int>> out;
   for (int id = 0; id < (int)insts_.size(); ++id) {
     const Inst& in = insts_[id];
     if (!in.live || in.failed) continue;
     const long long left = in.p.steps - done[id];
-    if (left <= 0) continue;
-    steps_of[id] = (int)std::min<long long>(left, window);
-    order.push_back({steps_of[id], id});
+    if (left > 0) out.push_back({(int)std::min<long long>(left, window), id});
   }
+  return out;
+}
+
+template <typename T>
+int Engine<T>::next_cut(int window, int* tile_depth, int* rows) const {
+  if (window < 1) return LE2D_EINVAL;
+  std::vector<long long> done(insts_.size());
+  for (size_t i = 0; i < insts_.size(); ++i) done[i] = insts_[i].done_steps;
+  const auto steps = window_steps(window, done);
+  if (steps.empty()) return LE2D_ESTATE;
+  const Cut cut = cut_window(steps);
+  *tile_depth = cut.tile_depth;
+  *rows = cut.rows;
+  return LE2D_OK;
+}
+
+template <typename T>
+typename Engine<T>::Window Engine<T>::plan_window(int window, const std::vector<long long>& done,
+                                                  const std::vector<int>& cur) const {
+  Window w;
+  std::vector<std::pair<int, int>> order = window_steps(window, done);  // then (work items in window, id)
+  std::vector<int> steps_of(insts_.size(), 0);
+  for (const auto& o : order) steps_of[o.second] = o.first;
   Cut cut;
   if (!order.empty()) cut = cut_window(order);
   w.tile_depth = cut.tile_depth;
@@ -916,6 +934,13 @@ int le2d_batch_run(le2d_batch* b, int window_steps, float* device_ms) {
   const int rc = b->eng->run_all(window_steps, device_ms);
   if (rc) fprintf(stderr, "le2d: le2d_batch_run: %s\n", le2d_strerror(rc));
   return rc;
+}
+
+int le2d_batch_set_strips(le2d_batch* b, int rows) { return b ? b->eng->set_seg_len(rows) : LE2D_EINVAL; }
+
+int le2d_batch_next_cut(const le2d_batch* b, int window_steps, int* out) {
+  if (!b || !out) return LE2D_EINVAL;
+  return b->eng->next_cut(window_steps, out, out + 1);
 }
 
 int le2d_batch_count(const le2d_batch* b) { return b ? b->eng->count() : 0; }

@@ -51,7 +51,7 @@ class Engine {
     int depth = 1;  // steps per work item of the batched kernel
     StepConsts<T> c;
     int nstrips = 0;
-    int seg_len = 0;  // tile height; 0: chosen for each window (window_rows)
+    int seg_len = 0;  // tile height; 0: chosen for each window (cut_window)
     bool live = false;
     int* fail = nullptr;     // failure word on the device (in the instance's arena block)
     bool failed = false;     // a dependency wait of one of its tiles gave up: no results
@@ -108,9 +108,15 @@ class Engine {
   void set_wait_ns(unsigned long long ns) { wait_ns_ = ns; }
   // Tile height and steps per work item for instances added afterwards (the autotuner's
   // trials); otherwise they come from the autotuner's table for the instance's size class,
-  // or the defaults (a height chosen for each window, batch_depth<T>()).
+  // or the defaults (a height chosen for each window, batch_depth<T>()).  A window with such an
+  // instance runs on strips.  Two steps at le_step_soa's far end read rows ny-7 and below, which
+  // have to lie in the last two tiles: kMinRows rows at least.
+  static constexpr int kMinRows = 8;
   int set_seg_len(int rows);
   int set_depth(int depth);
+  // How the next window of `window` steps is cut: *tile_depth steps per item on block tiles, or 0
+  // and strips, *rows high where the instance has no height of its own.
+  int next_cut(int window, int* tile_depth, int* rows) const;
   // Whether instances added afterwards take their tiles from the autotuner's table (default)
   // or the defaults.  The serving loop uses the defaults: the table is tuned for throughput
   // on a full batch, and its taller tiles lengthen each small instance's chain of steps.
@@ -133,6 +139,8 @@ class Engine {
   // done_steps / cur: each instance's steps so far and current buffer before the window.
   Window plan_window(int window, const std::vector<long long>& done_steps,
                      const std::vector<int>& cur) const;
+  // (steps, id) of the instances with steps left, in a window after done_steps.
+  std::vector<std::pair<int, int>> window_steps(int window, const std::vector<long long>& done_steps) const;
   // How a window in which instance steps[k].second runs steps[k].first time steps is cut: block
   // tiles of tile_depth steps per item, or strips, `rows` the tile height of the instances
   // without one of their own.
