@@ -292,6 +292,7 @@ int Engine<T>::alloc_instance(const le2d_problem& p, Inst& in) {
   const int out = strip_cols(batch_lanes<T>());
   in.nstrips = (p.nx + out - 1) / out;
   in.seg_len = std::min(seg, p.ny);
+  in.strips = seg_len_ != 0 || depth_set_ != 0;
   in.live = true;
   return LE2D_OK;
 }
@@ -409,6 +410,10 @@ int Engine<T>::read_failures(const std::vector<int>& ids) {
 // strips / block tiles at the depth picked): 8 instances with sides of 64 to 300 and 100 to 300
 // steps FP32 2.94 / 0.92, FP64 5.18 / 2.22; 32 of them 3.60 / 2.55 and 6.50 / 8.01 (strips kept);
 // the 24 above FP32 9.3 / 11.3 all on tiles, 8.5 with each window cut as it is faster.
+// A height from the autotuner's table is the instance's on strips; the table knows strips only, so
+// block tiles are weighed against it as against any other.  One tuned instance used to rule them
+// out for its whole window: 8 instances of 64 to 300 a side, 100 to 300 steps, one class tuned,
+// FP32 16.5 / 1.16 ms, FP64 33.9 / 3.5.
 template <typename T>
 typename Engine<T>::Cut Engine<T>::cut_window(const std::vector<std::pair<int, int>>& steps) const {
   constexpr bool f32 = sizeof(T) == 4;
@@ -420,12 +425,12 @@ typename Engine<T>::Cut Engine<T>::cut_window(const std::vector<std::pair<int, i
   constexpr int heights[] = {8, 12, 16, 24, 32, 48, 64};
   Cut best;
   double least = 1e300;
-  bool own = depth_set_ != 0 || stall_strips_;  // tile heights or depths of the instances' own: strips
+  bool strips = stall_strips_;
   for (int rows : heights) {
     double work = 0.0, chain = 0.0;
     for (const auto& o : steps) {
       const Inst& in = insts_[o.second];
-      own = own || in.seg_len != 0;
+      strips = strips || in.strips;
       const int l = std::min(in.seg_len ? in.seg_len : rows, in.p.ny);
       const int items = (o.first + in.depth - 1) / in.depth;
       work += (double)items * in.nstrips * ((in.p.ny + l - 1) / l) * (l + h);
@@ -437,7 +442,7 @@ typename Engine<T>::Cut Engine<T>::cut_window(const std::vector<std::pair<int, i
       best.rows = rows;
     }
   }
-  if (own || tile_blocks_ < 1) return best;
+  if (strips || tile_blocks_ < 1) return best;
   const BatchTileShape shape = batch_tile_shape<T>();
   for (int d = 1; d <= shape.max_depth; ++d) {
     double work = 0.0, chain = 0.0;

@@ -51,7 +51,8 @@ class Engine {
     int depth = 1;  // steps per work item of the batched kernel
     StepConsts<T> c;
     int nstrips = 0;
-    int seg_len = 0;  // tile height; 0: chosen for each window (cut_window)
+    int seg_len = 0;  // tile height on strips; 0: chosen for each window (cut_window)
+    bool strips = false;  // an explicit height or depth: its windows run on strips
     bool live = false;
     int* fail = nullptr;     // failure word on the device (in the instance's arena block)
     bool failed = false;     // a dependency wait of one of its tiles gave up: no results

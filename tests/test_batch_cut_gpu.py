@@ -51,3 +51,29 @@ def test_small_instances_take_block_tiles(prec):
         assert b.run(7)[0] == 0
         with pytest.raises(RuntimeError):
             b.next_cut(7)  # no steps left
+
+
+@pytest.mark.parametrize("prec", ["f", "d"])
+def test_tuned_class_keeps_block_tiles(prec):
+    """A tuned height is one for strips: it does not keep a window of small instances, tuned or not, off
+    block tiles."""
+    lib = capi.Lib(prec)
+    lib.batch_autotune_reset()
+    try:
+        lib.batch_autotune(100, 70)
+        todo = []
+        for k, (nx, ny) in enumerate(((100, 70), (90, 120), (200, 150), (65, 128), (128, 65), (40, 30))):
+            p = _problem(nx, ny, k)
+            g0 = np.random.default_rng(k).uniform(-1, 1, 5 * nx * ny).astype(lib.dtype)
+            todo.append((p, g0, _alone(lib, p, ST_AOS, g0, 0, 1000)[0]))
+        for strips in (0, 16):
+            with capi.Batch(lib, 1 << 28) as b:
+                if strips:
+                    assert b.set_strips(strips) == 0
+                ids = [b.add(b.problem(p), init=g0) for p, g0, _ in todo]
+                assert (b.next_cut(64)["tile_depth"] > 0) == (strips == 0)
+                assert b.run(64)[0] == 0
+                for i, (p, _, want) in zip(ids, todo):
+                    assert b.fields(i).tobytes() == want.tobytes(), (p.nx, p.ny, strips)
+    finally:
+        lib.batch_autotune_reset()
