@@ -74,7 +74,8 @@ int le2d_set_method(le_task *task, int method);
  * two warps of a tile that runs out (a fault, not a slow partner) is reported as
  * LE2D_ETIMEOUT at the next synchronisation (le2d_wait, le2d_download, le2d_sync_host). */
 int le2d_set_variant(le_task *task, int variant, int seg_len);
-/* out[8] = {variant, columns per lane, segment rows, strips, tiles, blocks,
+/* The strip plan (le2d_block_tiles says whether the task runs it).
+ * out[8] = {variant, columns per lane, segment rows, strips, tiles, blocks,
  * temporal-block depth, warps per tile (2: producer / consumer warp pair)}. */
 int le2d_get_plan(const le_task *task, int *out);
 /* Small grids on their default plan (no variant or segment length asked for, neither

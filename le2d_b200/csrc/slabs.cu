@@ -27,7 +27,7 @@
 // le_step_soa's far end (the last two rows read rows ny-5 and ny-4 instead of copies of row
 // ny-1) only affects the rows next to a grid's bottom: at a cut those are halo rows, and at
 // the last slab's bottom the slab's rows ny-5, ny-4 are the grid's.  So SoA tasks split too
-// (one step per launch, as whole SoA tasks).
+// (one step per launch; whole SoA tasks take two).
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -64,8 +64,8 @@ struct Slab {
   FusedPlan plan, plan1;
 };
 
-// Variant of each launch: FP32 two steps on warp pairs (one-step variant 2 for odd
-// remainders and SoA), FP64 one step (variant 15), as for whole tasks.
+// Variant of each launch: FP32 two steps on warp pairs, one-step variant 2 for odd remainders
+// and SoA; FP64 one step (variant 15).
 int two_step_variant() { return sizeof(T) == 4 ? 13 : 15; }
 int one_step_variant() { return sizeof(T) == 4 ? 2 : 15; }
 
