@@ -124,3 +124,26 @@ def test_result_pool():
     mixed sizes share the pieces, growth waits for two busy periods and ends at the bound."""
     out = _run(POOL)
     assert out == ["0", "0", "4", "4", "0", "1", "59", "1", "1", "1", "1"], out
+
+
+# FP64 default (148 SMs x 12 warps, 60 columns a strip), whole launches: us a step by segment length.
+WHOLE_F64 = {
+    (1000, 1000): {16: 30.8, 24: 41.3, 32: 38.9, 40: 47.1, 48: 55.3, 64: 71.0, 96: 102.4, 128: 133.2},
+    (1500, 1500): {16: 62.6, 24: 55.5, 32: 53.1, 40: 63.6, 48: 74.1, 64: 94.2, 96: 102.8, 128: 135.3},
+    (1800, 1800): {16: 74.6, 24: 90.1, 32: 74.0, 40: 88.5, 48: 76.3, 64: 98.0, 96: 104.5, 128: 135.3},
+    (2048, 2048): {16: 95.3, 24: 105.6, 32: 114.5, 40: 112.8, 48: 104.1, 64: 97.7, 96: 140.6, 128: 135.6},
+    (3000, 3000): {16: 187.1, 24: 188.0, 32: 182.9, 40: 182.2, 48: 202.6, 64: 221.7, 96: 196.9, 128: 248.4},
+    (4096, 4096): {16: 336.4, 24: 326.1, 32: 319.6, 40: 322.4, 48: 323.0, 64: 317.0, 96: 347.1, 128: 398.7},
+    (6000, 6000): {16: 729.5, 24: 720.4, 32: 693.1, 40: 691.4, 48: 686.8, 64: 662.8, 96: 676.2, 128: 659.7},
+    (8192, 2048): {16: 333.0, 24: 316.0, 32: 309.3, 40: 307.8, 48: 305.8, 64: 316.6, 96: 314.6, 128: 386.5},
+    (16384, 128): {16: 61.7, 24: 55.1, 32: 53.2, 40: 63.8, 48: 74.6, 64: 71.7, 96: 102.7, 128: 135.2},
+}
+
+
+def test_segment_model_of_whole_fp64_launches():
+    """The segment length picked for the FP64 default is within 5 % of the fastest one measured."""
+    calls = "".join(f'  std::printf("%d ", le2d::model_segment(le2d::kDefaultModelF64, {ny}, {(nx + 59) // 60}, '
+                    f'148 * 12, 16));\n' for nx, ny in WHOLE_F64)
+    out = _run('#include <cstdio>\n#include "segment_model.h"\nint main() {\n' + calls + "}\n")
+    for (size, times), seg in zip(WHOLE_F64.items(), map(int, out)):
+        assert times[seg] <= 1.05 * min(times.values()), (size, seg)
